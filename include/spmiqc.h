@@ -69,7 +69,8 @@ typedef struct spm_step_stats {
 /* Creates a context for an N^3 grid. Replaces the set-up of main_SPM.cpp:29-60
  * (LPsystParameter, get_kindex_all, My_mpi_fft_set_up, get_ksquare_local,
  * get_epmckt2_local, get_ikt2_local): k^2, G(k) and the preconditioner symbol
- * are evaluated inside the kernels, so no tables are built. stream may be NULL
+ * are evaluated inside the kernels (from N/2 + 1 factors per axis; FP32
+ * gradient chains read G from a table over K^2). stream may be NULL
  * (the legacy default stream). N must satisfy spm_supported_size(N). */
 int spm_ctx_create(int N, double L, double Tau, double Gamma, double dt, int precision,
                    void *stream, spm_ctx **out);
@@ -81,8 +82,12 @@ size_t spm_field_bytes(const spm_ctx *ctx);
 size_t spm_spectrum_bytes(const spm_ctx *ctx);
 const char *spm_status_str(int status);
 /* Tuning knobs (no counterpart in the reference; the analogue of FFTW's plan
- * choice, My_FFT.cpp:49-97). knob "plane_cps": 1 = plane kernels stage their
- * input in shared memory (one CTA per SM), 2 = direct loads, two CTAs per SM,
+ * choice, My_FFT.cpp:49-97). "plane_cps", "plane_xg" and "pencil_tc" concern
+ * the transforms, energies, gradients and gradient chains of FP32 contexts
+ * (and of the FP32 twins of mixed runs); FP64 ones, and the Hessian, preconditioner
+ * and force blocks of both precisions, run on kernels without such variants
+ * and take the values without effect. knob "plane_cps": 1 = plane kernels
+ * stage their input in shared memory (one CTA per SM), 2 = direct loads, two CTAs per SM,
  * 3 = direct loads, three CTAs per SM (fewer registers per thread), 4 = four
  * CTAs per SM for the exchanges through L2 of FP32 gradient chains (3
  * elsewhere), 5 = CTAs of 16 rows and 128 threads, four per SM, for gradient
@@ -117,8 +122,8 @@ const char *spm_status_str(int status);
 int spm_tune(spm_ctx *ctx, const char *knob, int value);
 int spm_tune_get(const spm_ctx *ctx, const char *knob);
 /* Autotuner (no counterpart in the reference): times chains of `steps`
- * gradient steps on a scratch field for each candidate schedule (plane_cps
- * 1/2/3 with fused chains, plane_cps 2 without, plane_xg 1/2/3 with plane_cps
+ * gradient steps on a scratch field for each candidate schedule (FP64: pdl 0
+ * and 1; FP32: plane_cps 1/2/3 with fused chains, plane_cps 2 without, plane_xg 1/2/3 with plane_cps
  * 2 and 3 on fused chains, plane_cps 4 for FP32, 5, 6; then pencil_tc 4 and
  * pdl 1 for the best of them), keeping a later candidate only if it is at least 1 % faster, and
  * keeps the fastest in the context; the choice is remembered per (device, N, precision), so later

@@ -95,9 +95,13 @@ extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_pla
   const Choice cands[] = {{2, 1, 0}, {3, 1, 0}, {1, 1, 0}, {2, 0, 0}, {2, 1, spm::kXgFwd | spm::kXgInv},
                           {3, 1, spm::kXgFwd | spm::kXgInv}, {2, 1, spm::kXgFwd}, {2, 1, spm::kXgInv}};
   std::vector<Choice> all(std::begin(cands), std::end(cands));
+  // FP64 chains run on the tile passes, which only "pdl" concerns
+  if (c->prec == SPM_FP64) all.assign(1, Choice{c->plane_cps, c->fuse_planes, c->plane_xg, c->pencil_tc});
   if (c->prec == SPM_FP32) all.push_back({4, 1, spm::kXgFwd | spm::kXgInv});  // four CTAs per SM
-  all.push_back({5, 1, spm::kXgFwd | spm::kXgInv});  // 16-row CTAs, four per SM
-  all.push_back({6, 1, spm::kXgFwd | spm::kXgInv});  // the same, fused pass pipelined over planes
+  if (c->prec == SPM_FP32) {
+    all.push_back({5, 1, spm::kXgFwd | spm::kXgInv});  // 16-row CTAs, four per SM
+    all.push_back({6, 1, spm::kXgFwd | spm::kXgInv});  // the same, fused pass pipelined over planes
+  }
   // best of three timed chains of `steps` gated steps with the candidate's knobs
   auto time_it = [&](const Choice &cand, float &t) -> int {
     c->plane_cps = cand.plane_cps;
@@ -137,7 +141,7 @@ extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_pla
   }
   // then the pencil tile width for the best schedule: 4-column tiles (several
   // CTAs per SM) if they are at least 1 % faster
-  if (rc == SPM_OK) {
+  if (rc == SPM_OK && c->prec == SPM_FP32) {
     Choice narrow = best;
     narrow.pencil_tc = 4;
     float t = 1e30f;

@@ -78,7 +78,19 @@ template <class T2> __device__ __forceinline__ T2 cmul(T2 a, T2 b) {
 template <class T2> __device__ __forceinline__ T2 cmulc(T2 a, T2 b) {  // a * conj(b)
   return {fma_rn(a.x, b.x, mul_rn(a.y, b.y)), fma_rn(a.y, b.x, -mul_rn(a.x, b.y))};
 }
-template <class T2> __device__ __forceinline__ T2 cconj(T2 a) { return {a.x, -a.y}; }
+// -a if the flag is set: a sign-bit flip, off the floating-point pipes.
+__device__ __forceinline__ double flip_if(double a, int flag) {
+  return __hiloint2double(__double2hiint(a) ^ (flag << 31), __double2loint(a));
+}
+__device__ __forceinline__ float flip_if(float a, int flag) {
+  return __int_as_float(__float_as_int(a) ^ (flag << 31));
+}
+template <class T2> __device__ __forceinline__ T2 flip_if(T2 a, int flag) {
+  return {flip_if(a.x, flag), flip_if(a.y, flag)};
+}
+template <class T2> __device__ __forceinline__ T2 shfl_xor(T2 a, int mask) {
+  return {__shfl_xor_sync(0xffffffffu, a.x, mask), __shfl_xor_sync(0xffffffffu, a.y, mask)};
+}
 template <class T2, class S> __device__ __forceinline__ T2 cscale(T2 a, S s) {
   return {a.x * s, a.y * s};
 }
@@ -218,6 +230,10 @@ template <class X, class = void> struct HasFacc : std::false_type {};
 template <class X> struct HasFacc<X, std::void_t<decltype(X::FACC)>> : std::bool_constant<X::FACC> {};
 template <class T, class X> constexpr bool use_facc() { return sizeof(T) == 4 && HasFacc<X>::value; }
 
+template <int NR, unsigned MAXM, int NA> __device__ __forceinline__ void acc_init(double (&a)[NA]) {
+#pragma unroll
+  for (int r = 0; r < NA; r++) a[r] = ((MAXM >> r) & 1u) ? -1.0e308 : 0.0;
+}
 template <int NR, unsigned MAXM> __device__ __forceinline__ void facc_init(float (&a)[NR]) {
 #pragma unroll
   for (int r = 0; r < NR; r++) a[r] = ((MAXM >> r) & 1u) ? -3.0e38f : 0.0f;
@@ -298,6 +314,9 @@ __device__ __forceinline__ bool grid_reduce(double (&acc)[NR], double *scratch, 
 // the CTA's error word and reports failure instead of spinning forever.
 __device__ __forceinline__ uint32_t smem_u32(const void *ptr) {
   return (uint32_t)__cvta_generic_to_shared(ptr);
+}
+__device__ __forceinline__ unsigned char *smem_base128(unsigned char *raw) {
+  return raw + ((128u - (smem_u32(raw) & 127u)) & 127u);
 }
 // Programmatic dependent launch. A kernel launched with the programmatic
 // stream-serialisation attribute may be set up while the previous kernel of
@@ -395,6 +414,19 @@ __device__ __forceinline__ float2 ld_stream(const float2 *p, uint64_t pol) {
   asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
   return v;
 }
+// A value of a state spectrum that the same kernel overwrites (volatile, as the
+// stores: a thread's loads and stores keep their order, so callers batch their
+// loads).
+__device__ __forceinline__ double2 ld_state(const double2 *p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 ld_state(const float2 *p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ void st_stream(double2 *p, double2 v, uint64_t pol) { st_keep(p, v, pol); }
 __device__ __forceinline__ void st_stream(float2 *p, float2 v, uint64_t pol) { st_keep(p, v, pol); }
 
@@ -459,6 +491,7 @@ struct ModelC {
   double Tau, Gamma, dt;
   double invL;     // 1/L, the reference's projection entry (Initialization.cpp:35-38)
   double inv_n3;   // 1/N^3
+  double fscale;   // 1/(2 N^3): scale of a forward transform by the tile passes (class_fwd keeps a factor 2)
   double n3;
   double G0;       // G(k = 0)
   double ikt0;     // 1/(G0 + |Tau| + 0.02)
@@ -471,10 +504,6 @@ struct ModelC {
 enum FlowWord { FW_GO = 0, FW_PENDING = 1, FW_ITER = 2, FW_ERR = 4 };
 
 struct KParams {
-  // Tensor maps of the strided inputs: tmi[b] over p.in[b], tms[b] over p.st[b]
-  // (filled by the launcher for the kernels that stage through TMA).
-  CUtensorMap tmi[kMaxBatch];
-  CUtensorMap tms[kMaxBatch];
   ModelC m;
   const void *in[kMaxBatch];
   void *out[kMaxBatch];
@@ -488,40 +517,96 @@ struct KParams {
   double *scal;         // [nb][kScal]
   int *flow;            // grad-flow control words (or null)
   double *stats;        // grad-flow per-step records (or null)
-  const double4 *gtab;  // per K^2 = Kx^2+Ky^2+Kz^2: {G, 1/(1+dt G), 1/(G+|Tau|+0.02), 1/(1+G)}
+  const double2 *gtab;  // symbol factors per |K| (pair_symbol)
   int *err;             // set when a bounded wait timed out
-  void *xg;             // plane kernels with XG: global exchange areas, xg_regions x xg_cap CTAs x PLANE_UNITS complex
-  int xg_cap;
-  int xg_regions;
+  int st_tiled, sto_tiled;  // pencil: the state read / written is in tile order (state_index)
   int nb;
   // Launches that batch independent instances of one grid size (gradient
   // chains of a batched relaxation) set `batched`: field b then takes its
-  // model, symbol table, flow words and step records from the arrays below
+  // model, symbol factors, flow words and step records from the arrays below
   // instead of m, gtab, flow and stats.
   int batched;
   ModelC mb[kMaxBatch];
-  const double4 *gtabs[kMaxBatch];
+  const double2 *gtabs[kMaxBatch];
   int *flows[kMaxBatch];
   double *statss[kMaxBatch];
 };
 
+// Parameters of the cluster passes (fft_kernels.cuh).
+struct KParamsC : KParams {
+  // Tensor maps of the strided inputs: tmi[b] over p.in[b], tms[b] over p.st[b]
+  // (filled by the launcher for the kernels that stage through TMA).
+  CUtensorMap tmi[kMaxBatch];
+  CUtensorMap tms[kMaxBatch];
+  const double2 *symtab;            // per K^2 = Kx^2+Ky^2+Kz^2: {G, 1/(1+dt G)}
+  const double2 *symtabs[kMaxBatch];  // (batched)
+  void *xg;             // global exchange areas, xg_regions x xg_cap CTAs x PLANE_UNITS complex
+  int xg_cap;
+  int xg_regions;
+};
+
 // Per-field views of the model, symbols, flow words and records (see `batched`).
 __device__ __forceinline__ const ModelC &model(const KParams &p, int b) { return p.batched ? p.mb[b] : p.m; }
-__device__ __forceinline__ const double4 *gtab_of(const KParams &p, int b) { return p.batched ? p.gtabs[b] : p.gtab; }
+__device__ __forceinline__ const double2 *gtab_of(const KParams &p, int b) { return p.batched ? p.gtabs[b] : p.gtab; }
+__device__ __forceinline__ const double2 *symtab_of(const KParamsC &p, int b) {
+  return p.batched ? p.symtabs[b] : p.symtab;
+}
 __device__ __forceinline__ int *flow_of(const KParams &p, int b) { return p.batched ? p.flows[b] : p.flow; }
 __device__ __forceinline__ double *stats_of(const KParams &p, int b) { return p.batched ? p.statss[b] : p.stats; }
 
-// Spectral symbols of wave vector (Kx, Ky, Kz) from the per-context table.
-__device__ __forceinline__ double4 symbols(const KParams &p, int Kx, int Ky, int Kz, int b = 0) {
-  const double2 *t = reinterpret_cast<const double2 *>(gtab_of(p, b)) + 2 * (Kx * Kx + Ky * Ky + Kz * Kz);
-  const double2 a = __ldg(t), c = __ldg(t + 1);
-  return make_double4(a.x, a.y, c.x, c.y);
+__device__ __forceinline__ bool flow_stopped(const KParams &p, int b) {
+  const int *f = flow_of(p, b);
+  return f != nullptr && *((volatile const int *)f + FW_GO) == 0;
+}
+// The step's stop is armed (FW_PENDING, set by its pencil pass before launch).
+__device__ __forceinline__ bool flow_pending(const KParams &p, int b) {
+  const int *f = flow_of(p, b);
+  return f != nullptr && *((volatile const int *)f + FW_PENDING) != 0;
 }
 
-// Half `h` of the symbols at K^2 (h = 0: {G, 1/(1+dt G)}, h = 1: {1/(G+|Tau|+0.02), 1/(1+G)}).
-__device__ __forceinline__ double2 symbols_half(const KParams &p, int k2, int h, int b = 0) {
-  return __ldg(reinterpret_cast<const double2 *>(gtab_of(p, b)) + 2 * k2 + h);
+// Pair kernel G(k^2) (Initialization.cpp:150-166) of a wave vector from the
+// per-axis factors {exp(-k_i^2 / (2 s^2)), k_i^2}, k_i = K_i / L, whose
+// product and sum over the axes give exp(-k^2 / (2 s^2)) and k^2: about nine
+// FP64 operations a point, where a table over K^2 costs a scattered lookup
+// (or, staged per tile, half as many 16-byte entries as the tile has points).
+// FP32 kernels evaluate it in FP64 too: near |k| = 1 the polynomial's terms
+// cancel to a hundredth of their size.
+__device__ __forceinline__ double pair_symbol(double2 a, double2 b) {
+  const double e = a.x * b.x, k2 = a.y + b.y;
+  const double q = fma(k2, fma(k2, fma(k2, fma(k2, 13.999261011773505, -38.839451762550148), 37.445683882581790),
+                               -14.949858723012090),
+                       1.969182919080340);
+  return fma(e, q, 0.08);
 }
+
+// 1 / x for normal x: the hardware's approximate reciprocal and two
+// Newton-Raphson steps, y <- y + y (1 - x y), each squaring the relative error
+// (2^-20 -> below 2^-52). No special cases: __drcp_rn's checks and slow-path
+// branches took 15 of the 256^3 gradient pencil's 157 us.
+__device__ __forceinline__ double fast_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// The symbols of a spectral point as the pencil operators see them, and the
+// scale of the forward values: evaluated by the tile passes, read from a table
+// by the cluster passes.
+struct SymFn {
+  double g;
+  __device__ double G() const { return g; }
+  __device__ double step(const ModelC &m) const { return fast_rcp(fma(m.dt, g, 1.0)); }  // 1/(1 + dt G)
+  __device__ double prec(const ModelC &m) const { return fast_rcp(g + fabs(m.Tau) + 0.02); }
+  __device__ double force() const { return fast_rcp(1.0 + g); }
+  __device__ static double scale(const ModelC &m) { return m.fscale; }
+};
+struct SymTab {
+  double2 v;
+  __device__ double G() const { return v.x; }
+  __device__ double step(const ModelC &) const { return v.y; }
+  __device__ static double scale(const ModelC &m) { return m.inv_n3; }
+};
 
 // Signed wave number of index i on an N grid (Initialization.cpp:97-107).
 __device__ __forceinline__ int wave(int i, int N) { return i < N / 2 ? i : i - N; }

@@ -1,4 +1,7 @@
-// The three streaming passes of a fused pseudo-spectral step on an N^3 grid.
+// The three streaming passes of a fused pseudo-spectral step on an N^3 grid with
+// the whole y transform in the plane passes, for FP32 gradient chains,
+// transforms, energies and gradients (cluster_impl.cuh says why these do not run
+// on the tile passes).
 //
 //   plane_fwd : thread-block clusters of CL = N/32 CTAs, each cluster looping
 //               over x-planes. Each CTA takes 32 z-rows of the real field,
@@ -25,6 +28,7 @@
 #include "fft_core.cuh"
 
 namespace spm {
+namespace clu {
 
 template <int N> struct Geo {
   static_assert(N % 32 == 0 && N >= 32 && N <= 256, "grid size must be a multiple of 32 in [32, 256]");
@@ -93,19 +97,6 @@ template <int N, class T, int TC = 8> constexpr size_t pencil_smem(int stages, b
   return pencil_smem_n<N, T, TC>(stages, pencil_sym_bufs<N, T, TC>(stages, sym));
 }
 
-__device__ __forceinline__ unsigned char *smem_base128(unsigned char *raw) {
-  return raw + ((128u - (smem_u32(raw) & 127u)) & 127u);
-}
-
-__device__ __forceinline__ bool flow_stopped(const KParams &p, int b) {
-  const int *f = flow_of(p, b);
-  return f != nullptr && *((volatile const int *)f + FW_GO) == 0;
-}
-// The step's stop is armed (FW_PENDING, set by its pencil pass before launch).
-__device__ __forceinline__ bool flow_pending(const KParams &p, int b) {
-  const int *f = flow_of(p, b);
-  return f != nullptr && *((volatile const int *)f + FW_PENDING) != 0;
-}
 
 // This CTA's global exchange area in region e (e = 0: inverse exchange, 1:
 // forward; the software-pipelined fused pass also uses 2 and 3, a second
@@ -115,7 +106,7 @@ __device__ __forceinline__ bool flow_pending(const KParams &p, int b) {
 template <int N, class T, int RW = kRows, int R = 2> struct XgAreas {
   c2<T> *own[R] = {};
   const c2<T> *first[R] = {};
-  __device__ XgAreas(const KParams &p, int rank) {
+  __device__ XgAreas(const KParamsC &p, int rank) {
     if (p.xg == nullptr) return;
     constexpr size_t U = (size_t)RW * (N / 2);
     const size_t region = (size_t)p.xg_cap * Geo<N>::PLANE_UNITS;
@@ -463,7 +454,7 @@ template <int N, class T> __device__ __forceinline__ void plane_twiddles(const K
 // in shared memory with a bulk copy; 2 has no stage (half the shared memory,
 // so two CTAs share an SM) and loads its rows straight from global memory.
 template <int N, class T, class Pro, int CPS, int XG = 0, int RW = kRows>
-__global__ void __launch_bounds__(8 * RW, CPS) plane_fwd_kernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(8 * RW, CPS) plane_fwd_kernel(const __grid_constant__ KParamsC p) {
   using G = Geo<N>;
   using T2 = c2<T>;
   using P = Plane<N, T, RW>;
@@ -571,8 +562,8 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_fwd_kernel(const __grid_con
 // Stages: [A (if FI)][S (if SI)], each 2 rows x N x 8 columns, [row][x][cc].
 template <int N, class T, class Op, int TC = 8>
 __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
-                                  pencil_min_ctas<N, T, TC>((Op::FI ? 1 : 0) + (Op::SI ? 1 : 0), Op::SYM >= 0))
-    pencil_kernel(const __grid_constant__ KParams p) {
+                                  pencil_min_ctas<N, T, TC>((Op::FI ? 1 : 0) + (Op::SI ? 1 : 0), Op::SYM))
+    pencil_kernel(const __grid_constant__ KParamsC p) {
   using G = Geo<N>;
   using PG = PencilGeo<N, TC>;
   using T2 = c2<T>;
@@ -608,16 +599,16 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
   // buffers they start at the top of the previous tile, with one once the
   // previous tile's point operator is done. Tiles with t = 0 (rows 0 and
   // N/2) read the table.
-  constexpr bool USE_SYM = Op::SYM >= 0;
+  constexpr bool USE_SYM = Op::SYM;
   constexpr int KXS = N / 2 + 1, SYMN = PG::SYMN;
   constexpr int SYMB = pencil_sym_bufs<N, T, TC>(NST, USE_SYM);
   auto sym_stage = [&](int tl, double2 *dst) {
     const int tt = tl / NCH, cz = (tl % NCH) * TC;
-    const double2 *g = reinterpret_cast<const double2 *>(gtab_of(p, b)) + (USE_SYM ? Op::SYM : 0);
+    const double2 *g = symtab_of(p, b);
     for (int e = tid; e < SYMN; e += TH) {
       const int row = e / KXS, a = e - row * KXS;
       const int kz = row < TC ? cz + row : N / 2;
-      cp_async16(dst + e, g + 2 * (a * a + tt * tt + kz * kz));
+      cp_async16(dst + e, g + (a * a + tt * tt + kz * kz));
     }
   };
   // this tile's copies complete (with two buffers the next tile's may not)
@@ -675,12 +666,12 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
       __syncthreads();
     }
     // symbols of (Kx, Ky, Kz) for kz row `row` of the tile (TC: kz = N/2)
-    auto sym_at = [&](int Kx, int Ky, int Kz, int row) -> double2 {
+    auto sym_at = [&](int Kx, int Ky, int Kz, int row) -> SymTab {
       if constexpr (!USE_SYM) {
-        return double2{0.0, 0.0};
+        return SymTab{};
       } else {
-        if (t != 0) return sym_cur[row * KXS + (Kx < 0 ? -Kx : Kx)];
-        return symbols_half(p, Kx * Kx + Ky * Ky + Kz * Kz, Op::SYM, b);
+        if (t != 0) return SymTab{sym_cur[row * KXS + (Kx < 0 ? -Kx : Kx)]};
+        return SymTab{__ldg(symtab_of(p, b) + Kx * Kx + Ky * Ky + Kz * Kz)};
       }
     };
 
@@ -826,7 +817,7 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
 // CPS as for plane_fwd: 1 stages the next plane's columns with a tensor copy,
 // 2 loads them straight from global memory (two CTAs per SM).
 template <int N, class T, class Epi, int CPS, int XG = 0, int RW = kRows>
-__global__ void __launch_bounds__(8 * RW, CPS) plane_inv_kernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(8 * RW, CPS) plane_inv_kernel(const __grid_constant__ KParamsC p) {
   using G = Geo<N>;
   using T2 = c2<T>;
   using P = Plane<N, T, RW>;
@@ -926,7 +917,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_kernel(const __grid_con
 // step. Direct loads; CPS (2, 3 or 4) CTAs per SM, the layout of plane_fwd's
 // direct variant.
 template <int N, class T, class Epi, class Pro, int CPS, int XG = 0, int RW = kRows>
-__global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_kernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_kernel(const __grid_constant__ KParamsC p) {
   using G = Geo<N>;
   using T2 = c2<T>;
   using P = Plane<N, T, RW>;
@@ -1053,7 +1044,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_kernel(const __grid
 // plane_inv_fwd, so results are identical. The stopping step (FW_PENDING)
 // runs the inverse half only, as plane_inv_fwd does.
 template <int N, class T, class Epi, class Pro, int CPS, int RW>
-__global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_pipe_kernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_pipe_kernel(const __grid_constant__ KParamsC p) {
   using G = Geo<N>;
   using T2 = c2<T>;
   using P = Plane<N, T, RW>;
@@ -1193,4 +1184,5 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_pipe_kernel(const _
   }
 }
 
+}  // namespace clu
 }  // namespace spm

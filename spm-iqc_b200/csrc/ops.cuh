@@ -2,7 +2,7 @@
 // reference's hot-path routines. Each policy cites the SPM-IQC code it follows.
 #pragma once
 
-#include "fft_kernels.cuh"
+#include "fft_core.cuh"
 
 namespace spm {
 
@@ -166,12 +166,13 @@ template <class T> struct ProHisd {
 // Forward transform with the reference's 1/N^3 (My_FFT.cpp:9-13): store only.
 template <class T> struct OpFwd {
   static constexpr bool FI = true, SI = false, SO = true, INV = false, LIN = true;
-  static constexpr int SYM = -1;
+  static constexpr bool SYM = false;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &p, int, int, int, int, double2, c2<T> f, c2<T>, c2<T> &so,
+  template <class S>
+  __device__ static void point(const KParams &p, int, int, int, int, S, c2<T> f, c2<T>, c2<T> &so,
                                c2<T> &, double (&)[1], double) {
-    so = cscale(f, (T)p.m.inv_n3);
+    so = cscale(f, (T)S::scale(p.m));
   }
   __device__ static void fin(const KParams &, int, const double (&)[1]) {}
 };
@@ -179,10 +180,11 @@ template <class T> struct OpFwd {
 // Backward transform of a stored spectrum (My_FFT.cpp:15-21): inverse only.
 template <class T> struct OpInv {
   static constexpr bool FI = false, SI = true, SO = false, INV = true, LIN = true;
-  static constexpr int SYM = -1;
+  static constexpr bool SYM = false;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &, int, int, int, int, double2, c2<T>, c2<T> s, c2<T> &, c2<T> &inv,
+  template <class S>
+  __device__ static void point(const KParams &, int, int, int, int, S, c2<T>, c2<T> s, c2<T> &, c2<T> &inv,
                                double (&)[1], double) {
     inv = s;
   }
@@ -198,17 +200,18 @@ template <class T> struct OpInv {
 // FP32 rounding already), then join the FP64 totals.
 template <class T> struct OpGrad {
   static constexpr bool FI = true, SI = true, SO = true, INV = true, LIN = false;
-  static constexpr int SYM = 0;  // {G, 1/(1 + dt G)}
+  static constexpr bool SYM = true;
   static constexpr int NR = 3;
   static constexpr unsigned MAXM = 0x2;
   static constexpr bool FACC = true;
-  template <class A>
-  __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, double2 sy, c2<T> f, c2<T> s,
+  template <class S, class A>
+  __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T> s,
                                c2<T> &so, c2<T> &inv, A (&acc)[3], double w) {
-    const A G = (A)sy.x;
-    const T dt = (T)model(p, b).dt;
-    const c2<T> fh = cscale(f, (T)model(p, b).inv_n3);
-    const T iden = (T)sy.y;  // 1 / (1 + dt G)
+    const ModelC &m = model(p, b);
+    const A G = (A)sy.G();
+    const T dt = (T)m.dt;
+    const c2<T> fh = cscale(f, (T)S::scale(m));
+    const T iden = (T)sy.step(m);  // 1 / (1 + dt G)
     c2<T> u1 = {(dt * fh.x + s.x) * iden, (dt * fh.y + s.y) * iden};
     const bool k0 = (Kx == 0 && Ky == 0 && Kz == 0);
     if (k0) u1 = c2<T>{0, 0};
@@ -253,13 +256,13 @@ template <class T> struct OpGrad {
 // mode is kept) or, with ZERO_DC, for ngrad_cam (LPsrc.cpp:133-142).
 template <class T, bool ZERO_DC> struct OpGmul {
   static constexpr bool FI = true, SI = false, SO = false, INV = true, LIN = false;
-  static constexpr int SYM = 0;
+  static constexpr bool SYM = true;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, double2 sy, c2<T> f, c2<T>, c2<T> &,
+  template <class S>
+  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T>, c2<T> &,
                                c2<T> &inv, double (&)[1], double) {
-    const T g = (T)sy.x;
-    inv = cscale(cscale(f, (T)p.m.inv_n3), g);
+    inv = cscale(cscale(f, (T)S::scale(p.m)), (T)sy.G());
     if (ZERO_DC && Kx == 0 && Ky == 0 && Kz == 0) inv = c2<T>{0, 0};
   }
   __device__ static void fin(const KParams &, int, const double (&)[1]) {}
@@ -268,13 +271,14 @@ template <class T, bool ZERO_DC> struct OpGmul {
 // Preconditioner symbol 1/(G + |Tau| + 0.02) (Initialization.cpp:123-129, LOBPCG.cpp:175-179).
 template <class T> struct OpPrecond {
   static constexpr bool FI = true, SI = false, SO = false, INV = true, LIN = false;
-  static constexpr int SYM = 1;  // {1/(G + |Tau| + 0.02), 1/(1 + G)}
+  static constexpr bool SYM = true;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, double2 sy, c2<T> f, c2<T>, c2<T> &,
+  template <class S>
+  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T>, c2<T> &,
                                c2<T> &inv, double (&)[1], double) {
-    const T ik = (T)sy.x;  // 1 / (G + |Tau| + 0.02)
-    inv = cscale(cscale(f, (T)p.m.inv_n3), ik);
+    const T ik = (T)sy.prec(p.m);  // 1 / (G + |Tau| + 0.02)
+    inv = cscale(cscale(f, (T)S::scale(p.m)), ik);
   }
   __device__ static void fin(const KParams &, int, const double (&)[1]) {}
 };
@@ -284,14 +288,15 @@ template <class T> struct OpPrecond {
 // spectrum of the tangent.
 template <class T> struct OpForce {
   static constexpr bool FI = true, SI = true, SO = false, INV = true, LIN = false;
-  static constexpr int SYM = 1;
+  static constexpr bool SYM = true;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, double2 sy, c2<T> f, c2<T> s, c2<T> &,
+  template <class S>
+  __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T> s, c2<T> &,
                                c2<T> &inv, double (&)[1], double) {
-    const T iden = (T)sy.y;  // 1 / (1 + G)
+    const T iden = (T)sy.force();  // 1 / (1 + G)
     const T sc = (T)scal_of(p, b)[SC_S];
-    const c2<T> fh = cscale(f, (T)p.m.inv_n3);
+    const c2<T> fh = cscale(f, (T)S::scale(p.m));
     inv = c2<T>{(fh.x - sc * s.x) * iden, (fh.y - sc * s.y) * iden};
     if (Kx == 0 && Ky == 0 && Kz == 0) inv = c2<T>{0, 0};
   }
@@ -303,16 +308,16 @@ template <class T> struct OpForce {
 // field is taken as given (||d|| := 1), for force steps along a caller's v.
 template <class T, bool NORM = true> struct OpTangent {
   static constexpr bool FI = true, SI = false, SO = true, INV = true, LIN = false;
-  static constexpr int SYM = 0;
+  static constexpr bool SYM = true;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, double2 sy, c2<T> f, c2<T>, c2<T> &so,
+  template <class S>
+  __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T>, c2<T> &so,
                                c2<T> &inv, double (&)[1], double) {
     const T inrm = NORM ? (T)(1.0 / sqrt(scal_of(p, b)[SC_NRM2])) : (T)1;
-    const c2<T> v = cscale(cscale(f, (T)p.m.inv_n3), inrm);
+    const c2<T> v = cscale(cscale(f, (T)S::scale(p.m)), inrm);
     so = v;
-    const T g = (T)sy.x;
-    inv = (Kx == 0 && Ky == 0 && Kz == 0) ? c2<T>{0, 0} : cscale(v, g);
+    inv = (Kx == 0 && Ky == 0 && Kz == 0) ? c2<T>{0, 0} : cscale(v, (T)sy.G());
   }
   __device__ static void fin(const KParams &, int, const double (&)[1]) {}
 };
@@ -321,14 +326,15 @@ template <class T, bool NORM = true> struct OpTangent {
 // the imaginary part set to 0, as the reference does, and x'^_0 = 0.
 template <class T> struct OpHisd {
   static constexpr bool FI = true, SI = false, SO = false, INV = true, LIN = false;
-  static constexpr int SYM = 0;
+  static constexpr bool SYM = true;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, double2 sy, c2<T> f, c2<T>, c2<T> &,
+  template <class S>
+  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T>, c2<T> &,
                                c2<T> &inv, double (&)[1], double) {
     const T beta = (T)p.m.factor;
-    const T den = (T)1 + beta * (T)sy.x;
-    inv = c2<T>{f.x * (T)p.m.inv_n3 / den, (T)0};
+    const T den = (T)1 + beta * (T)sy.G();
+    inv = c2<T>{f.x * (T)S::scale(p.m) / den, (T)0};
     if (Kx == 0 && Ky == 0 && Kz == 0) inv = c2<T>{0, 0};
   }
   __device__ static void fin(const KParams &, int, const double (&)[1]) {}
@@ -337,12 +343,13 @@ template <class T> struct OpHisd {
 // E1 = 1/2 sum_k G |u_k|^2 of a stored spectrum (LPsrc.cpp:27-35): reduction only.
 template <class T> struct OpE1 {
   static constexpr bool FI = false, SI = true, SO = false, INV = false, LIN = false;
-  static constexpr int SYM = 0;
+  static constexpr bool SYM = true;
   static constexpr int NR = 1;
   static constexpr unsigned MAXM = 0;
-  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, double2 sy, c2<T>, c2<T> s, c2<T> &, c2<T> &,
+  template <class S>
+  __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, S sy, c2<T>, c2<T> s, c2<T> &, c2<T> &,
                                double (&acc)[1], double w) {
-    const double G = sy.x;
+    const double G = sy.G();
     acc[0] += w * 0.5 * G * ((double)s.x * (double)s.x + (double)s.y * (double)s.y);
   }
   __device__ static void fin(const KParams &p, int b, const double (&tot)[1]) {

@@ -82,8 +82,16 @@ KParams spm_params(const spm_ctx *c) {
   p.tickets = c->tickets;
   p.scal = c->scal;
   p.flow = c->gate;
-  p.gtab = reinterpret_cast<const double4 *>(c->gtab);
+  p.gtab = reinterpret_cast<const double2 *>(c->gtab);
   p.err = c->flow + FW_ERR;
+  return p;
+}
+
+KParamsC spm_params_c(const spm_ctx *c) {
+  KParamsC p;
+  std::memset(&p, 0, sizeof(p));
+  static_cast<KParams &>(p) = spm_params(c);
+  p.symtab = reinterpret_cast<const double2 *>(c->symtab);
   p.xg = c->xg;
   p.xg_cap = c->xg_cap;
   p.xg_regions = c->xg ? spm::kXgRegions : 0;
@@ -95,7 +103,7 @@ KParams spm_params(const spm_ctx *c) {
 // min(SMs x CTAs per SM, N x CL) CTAs, the CTAs per SM bounded by the plane
 // kernels' shared memory and 8 blocks of 256 threads.
 int spm_ensure_xg(spm_ctx *c) {
-  if (!c->plane_xg || c->xg) return SPM_OK;
+  if (!c->plane_xg || c->xg || c->prec != SPM_FP32) return SPM_OK;  // only the cluster passes exchange
   int sms = 0, smem_sm = 0;
   cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device);
@@ -116,28 +124,23 @@ int spm_ensure_xg(spm_ctx *c) {
   return SPM_OK;
 }
 
-int spm_ensure_scratch(spm_ctx *c, int nb) {
+int spm_ensure_scratch(spm_ctx *c, int nf) {
   SPM_TRY(spm_ensure_xg(c));
-  if (nb <= c->scratch_cap) return SPM_OK;
-  if (c->bufA) cudaFree(c->bufA);
-  if (c->bufB) cudaFree(c->bufB);
-  c->bufA = c->bufB = nullptr;
+  if (nf < 2) nf = 2;  // every chain of one field
+  if (nf <= c->scratch_cap) return SPM_OK;
+  cudaFree(c->buf);
+  c->buf = nullptr;
   c->scratch_cap = 0;
-  const size_t bytes = c->field_bytes * (size_t)nb;
-  cudaError_t e = cudaMalloc(&c->bufA, bytes);
-  if (e != cudaSuccess) return spm_fail_cuda(e, "scratch A");
-  e = cudaMalloc(&c->bufB, bytes);
+  cudaError_t e = cudaMalloc(&c->buf, c->field_bytes * (size_t)nf);
   if (e != cudaSuccess) {
-    cudaFree(c->bufA);
-    c->bufA = nullptr;
-    return spm_fail_cuda(e, "scratch B");
+    c->buf = nullptr;
+    return spm_fail_cuda(e, "spectral scratch");
   }
-  c->scratch_cap = nb;
+  c->scratch_cap = nf;
   return SPM_OK;
 }
 
-char *spm_bufA(spm_ctx *c, int b) { return (char *)c->bufA + c->field_bytes * (size_t)b; }
-char *spm_bufB(spm_ctx *c, int b) { return (char *)c->bufB + c->field_bytes * (size_t)b; }
+char *spm_buf(spm_ctx *c, int i) { return (char *)c->buf + c->field_bytes * (size_t)i; }
 
 // ------------------------------------------------------------------ tensor maps
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -265,6 +268,7 @@ extern "C" int spm_ctx_create(int N, double L, double Tau, double Gamma, double 
   c->L = L;
   c->m.invL = 1.0 / L;
   c->m.inv_n3 = 1.0 / n3;
+  c->m.fscale = 0.5 / n3;
   c->m.n3 = n3;
   {  // G(0) and the preconditioner symbol at k = 0 (Initialization.cpp:123-166)
     const double ph = 0.568809, s2 = ph * ph, k2 = 0.0;
@@ -294,14 +298,34 @@ extern "C" int spm_ctx_create(int N, double L, double Tau, double Gamma, double 
                    cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { spm_ctx_destroy(c); return spm_fail_cuda(e, "twiddles"); }
   }
-  // Spectral symbols per K^2 = Kx^2 + Ky^2 + Kz^2 (every K in [-N/2, N/2)):
-  // G(k^2) with k^2 = K^2 / L^2 (get_GK, Initialization.cpp:150-166), the
-  // gradient-step factor 1/(1 + dt G) (LPsrc.cpp:64-67), the preconditioner
-  // symbol 1/(G + |Tau| + 0.02) (Initialization.cpp:123-129) and the force-step
-  // factor 1/(1 + G) (SPM.cpp:82-86).
+  // Factors of the pair kernel per axis (pair_symbol): {exp(-k^2 / (2 s^2)),
+  // k^2} with k = K / L for |K| = 0 .. N/2.
+  auto upload = [&](const std::vector<double> &tab, double **dev) {
+    cudaError_t e = cudaMalloc(dev, sizeof(double) * tab.size());
+    if (e == cudaSuccess) e = cudaMemcpy(*dev, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice);
+    return e;
+  };
   {
+    std::vector<double> tab(2 * (size_t)(N / 2 + 1));
+    const long double s2 = 0.568809L * 0.568809L, invL = 1.0L / (long double)L;
+    for (int K = 0; K <= N / 2; K++) {
+      const long double k2 = (long double)K * K * (invL * invL);
+      tab[2 * (size_t)K] = (double)expl(-0.5L * k2 / s2);
+      tab[2 * (size_t)K + 1] = (double)k2;
+    }
+    const cudaError_t e = upload(tab, &c->gtab);
+    if (e != cudaSuccess) {
+      spm_ctx_destroy(c);
+      return spm_fail_cuda(e, "symbol factors");
+    }
+  }
+  // FP32 contexts: spectral symbols per K^2 = Kx^2 + Ky^2 + Kz^2 (every K in
+  // [-N/2, N/2)) for the cluster passes: G(k^2) with k^2 = K^2 / L^2 (get_GK,
+  // Initialization.cpp:150-166) and the gradient-step factor 1/(1 + dt G)
+  // (LPsrc.cpp:64-67).
+  if (precision == SPM_FP32) {
     const int kmax = 3 * (N / 2) * (N / 2);
-    std::vector<double> tab(4 * (size_t)(kmax + 1));
+    std::vector<double> tab(2 * (size_t)(kmax + 1));
     const double ph = 0.568809, s2 = ph * ph, invL = 1.0 / L;
     for (int K2 = 0; K2 <= kmax; K2++) {
       const double k2 = (double)K2 * (invL * invL);
@@ -310,14 +334,10 @@ extern "C" int spm_ctx_create(int N, double L, double Tau, double Gamma, double 
                            (1.969182919080340 + -14.949858723012090 * k2 + 37.445683882581790 * k4 +
                             -38.839451762550148 * k6 + 13.999261011773505 * k8) +
                        0.08;
-      tab[4 * (size_t)K2 + 0] = G;
-      tab[4 * (size_t)K2 + 1] = 1.0 / (1.0 + dt * G);
-      tab[4 * (size_t)K2 + 2] = 1.0 / (G + std::fabs(Tau) + 0.02);
-      tab[4 * (size_t)K2 + 3] = 1.0 / (1.0 + G);
+      tab[2 * (size_t)K2 + 0] = G;
+      tab[2 * (size_t)K2 + 1] = 1.0 / (1.0 + dt * G);
     }
-    cudaError_t e = cudaMalloc(&c->gtab, sizeof(double) * tab.size());
-    if (e == cudaSuccess)
-      e = cudaMemcpy(c->gtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice);
+    const cudaError_t e = upload(tab, &c->symtab);
     if (e != cudaSuccess) {
       spm_ctx_destroy(c);
       return spm_fail_cuda(e, "symbol table");
@@ -354,8 +374,8 @@ extern "C" int spm_ctx_destroy(spm_ctx *c) {
   cudaFree(c->scal);
   cudaFree(c->flow);
   cudaFree(c->stats);
-  cudaFree(c->bufA);
-  cudaFree(c->bufB);
+  cudaFree(c->symtab);
+  cudaFree(c->buf);
   cudaFree(c->xg);
   cudaFree(c->host_phi);
   cudaFree(c->host_uhat);

@@ -37,8 +37,7 @@ struct spm_ctx {
   int *flow = nullptr;
   double *stats = nullptr;
   int stats_cap = 0;
-  void *bufA = nullptr;     // spectral scratch, scratch_cap fields
-  void *bufB = nullptr;
+  void *buf = nullptr;      // spectral scratch, scratch_cap fields
   int scratch_cap = 0;
   double *host_scal = nullptr;  // pinned
   int *host_flow = nullptr;     // pinned
@@ -47,7 +46,8 @@ struct spm_ctx {
   void *host_phi = nullptr;     // device copies used by the host-buffer entry points
   void *host_uhat = nullptr;
   int *gate = nullptr;          // flow words gating every launch of a solver chain (or null)
-  double *gtab = nullptr;       // spectral symbols per K^2 (4 doubles each)
+  double *gtab = nullptr;       // symbol factors per |K| (2 doubles each, pair_symbol)
+  double *symtab = nullptr;     // FP32 contexts: {G, 1/(1 + dt G)} per K^2 (cluster passes)
   std::vector<TmEntry> tmaps;   // tensor-map cache (most recent last)
   int plane_cps = 2;            // plane-kernel variant: CTAs per SM (1 staged; 2, 3 direct; 4 FP32 chains)
   int fuse_planes = 1;          // gradient chains use the fused inverse -> forward plane pass
@@ -69,11 +69,15 @@ inline bool spm_cancelled(const spm_ctx *c) { return c->cancel && *c->cancel; }
 int spm_fail(int status, const char *what);
 int spm_fail_cuda(cudaError_t e, const char *what);
 spm::KParams spm_params(const spm_ctx *c);
-int spm_ensure_scratch(spm_ctx *c, int nb);
+spm::KParamsC spm_params_c(const spm_ctx *c);  // for the cluster passes
+// Scratch for nf fields at least. A transform pass needs one per batched field, a
+// gradient chain two (its spectrum and the tiled u; the cluster passes, two
+// spectra).
+int spm_ensure_scratch(spm_ctx *c, int nf);
 // Allocates the global exchange areas when c->plane_xg asks for them.
 int spm_ensure_xg(spm_ctx *c);
-char *spm_bufA(spm_ctx *c, int b);
-char *spm_bufB(spm_ctx *c, int b);
+char *spm_buf(spm_ctx *c, int i);
+inline char *spm_buf2(spm_ctx *c, int b) { return spm_buf(c, b + 1); }  // second scratch of the cluster passes
 int spm_read_scal(spm_ctx *c, int nb);
 int spm_check_device_error(spm_ctx *c);
 int spm_flow_init(spm_ctx *c, cudaStream_t s);    // go = 1, iter = 0

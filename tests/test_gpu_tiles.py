@@ -1,0 +1,69 @@
+"""The tile passes (tile_kernels.cuh) at every grid size against the NumPy
+oracle: Hessian-product and preconditioner blocks in both precisions, and a
+gradient chain that stops inside (its tile-ordered spectrum goes back to the
+caller's array).
+
+Bars: FP64 1e-11 of the largest value (the parity bar of the other tests).
+FP32: a transform pair of N^3 points rounds each value about 2 log2(N^3) times;
+with errors of at most eps = 2^-24 per rounding and operands up to ~6 rms (a
+unit-variance random block) the bar is 6 * 2 * 3 log2(N) * 2^-24 of the rms,
+at most 1.8e-5 (N = 256)."""
+import numpy as np
+import pytest
+
+from conftest import rel
+from oracle import spmiqc_np as npo
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [32, 64, 96, 128, 160, 192, 256]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("N", SIZES)
+def test_blocks_match_oracle(cuda, N, prec):
+    import spmiqc
+    m = npo.Model(N, L=21.3, Tau=-0.013)
+    c = spmiqc.SpmContext(N, L=21.3, Tau=-0.013, precision=prec)
+    dt = np.float64 if prec == "fp64" else np.float32
+    rng = np.random.default_rng(N)
+    phi = (0.1 * rng.standard_normal((N, N, N))).astype(dt)
+    nb = 1 if N == 256 else 3
+    v = rng.standard_normal((nb, N, N, N)).astype(dt)
+    v[0] += dt(0.5)  # a mean, so the k = 0 modes matter
+    vd = cuda.from_numpy(v).cuda()
+    h = c.hv_cam(cuda.from_numpy(phi).cuda(), vd).cpu().numpy().astype(np.float64)
+    w = c.precond_camnew(vd).cpu().numpy().astype(np.float64)
+    for b in range(nb):
+        x = v[b].astype(np.float64)
+        for got, ref in ((h[b], m.hv(phi.astype(np.float64), x)), (w[b], m.precond(x))):
+            if prec == "fp64":
+                assert rel(got, ref) < 1e-11
+            else:
+                bar = 36 * np.log2(N) * 2.0 ** -24 * np.sqrt(np.mean(ref * ref))
+                assert np.max(np.abs(got - ref)) < bar
+    c.close()
+
+
+@pytest.mark.parametrize("N", SIZES)
+def test_chain_stopping_inside_returns_its_state(cuda, N):
+    """A flow that reaches tol_grad inside an enqueued chain leaves phi and uhat
+    of its last step: uhat = my_fft(phi), and both as a flow of exactly that
+    many steps gives them."""
+    import spmiqc
+    phi0 = npo.uniform_field(N, 77)
+    ctx = spmiqc.SpmContext(N, Tau=-0.02)
+
+    def flow(steps, tol):
+        p = cuda.from_numpy(phi0.copy()).cuda()
+        u = ctx.my_fft(p)
+        return ctx.get_min_u_F(p, u, steps, tol_grad=tol), p, u
+
+    probe, _, _ = flow(30, 0.0)
+    st, p, u = flow(400, float(probe[19, 2]))  # reached at step 20, inside the second chunk
+    assert len(st) == 20
+    _, q, w = flow(20, 0.0)
+    assert cuda.equal(p, q) and cuda.equal(u, w)
+    back = ctx.my_fft(p)
+    assert rel(back.cpu().numpy(), u.cpu().numpy()) < 1e-11
+    ctx.close()
