@@ -322,12 +322,14 @@ __device__ __forceinline__ unsigned char *smem_base128(unsigned char *raw) {
 // stream-serialisation attribute may be set up while the previous kernel of
 // its stream completes; the wait blocks until that kernel has completed and
 // its writes are visible, so every kernel launched that way runs this before
-// its first global-memory access (a no-op in a plain launch). No kernel
-// triggers its dependents early (griddepcontrol.launch_dependents): with the
-// trigger at the top of each kernel, CTAs of the next launch were placed on
-// the SMs as this grid's CTAs retired, and 256^3 gradient chains ran 20-25 %
-// slower.
+// its first access to data that an earlier kernel writes (a no-op in a plain
+// launch).
 __device__ __forceinline__ void grid_dep_sync() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next launch of the stream be placed from here on. Only for grids
+// that leave room on the device (KParams::trigger): with the trigger in
+// full-device grids, blocks of the next launch took the slots of this grid's
+// retiring blocks, and 256^3 gradient chains ran 20-25 % slower.
+__device__ __forceinline__ void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -521,6 +523,7 @@ struct KParams {
   int *err;             // set when a bounded wait timed out
   int st_tiled, sto_tiled;  // pencil: the state read / written is in tile order (state_index)
   int nb;
+  int trigger;          // tile kernels: the grid leaves room for the next launch (grid_dep_trigger)
   // Launches that batch independent instances of one grid size (gradient
   // chains of a batched relaxation) set `batched`: field b then takes its
   // model, symbol factors, flow words and step records from the arrays below

@@ -3,6 +3,8 @@
 // through the OpsTable of the context.
 #pragma once
 
+#include <algorithm>
+
 #include "cluster_impl.cuh"
 #include "launch.cuh"
 #include "tile_kernels.cuh"
@@ -15,25 +17,30 @@ namespace spm {
 // load), so the reductions' partial sums, and hence the results, do not
 // either. With pdl_on the launch is a programmatic dependent one: it may be set
 // up while the previous kernel of the stream finishes, and waits for it in
-// grid_dep_sync.
+// grid_dep_sync. Grids of at most half of the resident blocks (all but a few
+// of the batched ones up to 96^3) are launched that way in any case, and let the next
+// launch in as soon as they run: its blocks are then placed, with their
+// twiddles loaded, when this one completes.
 template <class Tag, class K>
-static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles, const KParams &p, int nb,
+static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles, const KParams &p0, int nb,
                         const char *what) {
   cudaError_t e = prepare<Tag>(kern, smem, c->device);
   if (e != cudaSuccess) return spm_fail_cuda(e, what);
-  static std::atomic<int> nblk[32] = {};
+  static std::atomic<int> resident[32] = {};
   const int dev = c->device < 32 ? c->device : 0;
-  int nbk = nblk[dev].load(std::memory_order_relaxed);
-  if (nbk == 0) {
+  int most = resident[dev].load(std::memory_order_relaxed);
+  if (most == 0) {
     int per_sm = 0, sms = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     if (e != cudaSuccess || per_sm < 1)
       return spm_fail_cuda(e != cudaSuccess ? e : cudaErrorInvalidConfiguration, what);
-    nbk = per_sm * sms < tiles ? per_sm * sms : tiles;
-    if (nbk > kPartStride) nbk = kPartStride;
-    nblk[dev].store(nbk, std::memory_order_relaxed);
+    most = per_sm * sms;
+    resident[dev].store(most, std::memory_order_relaxed);
   }
+  const int nbk = std::min({most, tiles, kPartStride});
+  KParams p = p0;
+  p.trigger = 2 * nbk * nb <= most;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nbk, nb, 1);
   cfg.blockDim = dim3(threads, 1, 1);
@@ -43,7 +50,7 @@ static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles,
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pdl_on(c) ? 1 : 0;  // the kernels begin with grid_dep_sync
+  cfg.numAttrs = pdl_on(c) || p.trigger ? 1 : 0;
   c->launches++;
   e = cudaLaunchKernelEx(&cfg, kern, p);
   return e == cudaSuccess ? 0 : spm_fail_cuda(e, what);

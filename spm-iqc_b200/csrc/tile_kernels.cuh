@@ -319,12 +319,13 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
   T2 *tw = reinterpret_cast<T2 *>(smem_raw);
   T2 *buf = tw + N;
   double *red = reinterpret_cast<double *>(buf + PG::UNITS + (PG::UNITS & 1));
+  load_twiddles<N, T>(p, tw);
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
   const int tid = threadIdx.x, b = blockIdx.y;
   const T *src = reinterpret_cast<const T *>(p.in[b]);
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
-  load_twiddles<N, T>(p, tw);
   double acc[Pro::NR > 0 ? Pro::NR : 1];
   acc_init<Pro::NR, Pro::MAXM>(acc);
   for (int tile = blockIdx.x; tile < PG::TILES; tile += gridDim.x) {
@@ -375,12 +376,13 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
   T2 *tw = reinterpret_cast<T2 *>(smem_raw);
   T2 *buf = tw + N;
   double *red = reinterpret_cast<double *>(buf + PG::UNITS + (PG::UNITS & 1));
+  load_twiddles<N, T>(p, tw);
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
   const int tid = threadIdx.x, b = blockIdx.y;
   const T2 *src = reinterpret_cast<const T2 *>(p.in[b]);
   T *outb = reinterpret_cast<T *>(p.out[b]);  // null: reductions only
-  load_twiddles<N, T>(p, tw);
   double acc[Epi::NR > 0 ? Epi::NR : 1];
   acc_init<Epi::NR, Epi::MAXM>(acc);
   __syncthreads();
@@ -434,7 +436,9 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
   T2 *tw = reinterpret_cast<T2 *>(smem_raw);
   T2 *buf = tw + N;
   double *red = reinterpret_cast<double *>(buf + PG::UNITS + (PG::UNITS & 1));
+  load_twiddles<N, T>(p, tw);
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
   // uniform over the grid: set by the pencil pass of this step, before launch
   const bool stop = flow_pending(p, blockIdx.y);
@@ -442,7 +446,6 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
   const T2 *src = reinterpret_cast<const T2 *>(p.in[b]);
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
   T *phi = reinterpret_cast<T *>(p.sto[b]);
-  load_twiddles<N, T>(p, tw);
   double acc_e[NE > 0 ? NE : 1], acc_p[NP > 0 ? NP : 1];
   acc_init<NE, Epi::MAXM>(acc_e);
   acc_init<NP, Pro::MAXM>(acc_p);
@@ -551,16 +554,17 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
   T2 *ex = tw + N;
   double2 *gx = reinterpret_cast<double2 *>(ex + PG::UNITS + (PG::UNITS & 1));  // symbol factors per |K|
   double *red = reinterpret_cast<double *>(gx + N / 2 + 1);
-  grid_dep_sync();
-  if (flow_stopped(p, blockIdx.y)) return;
   const int tid = threadIdx.x, b = blockIdx.y;
+  load_twiddles<N, T>(p, tw);
+  if constexpr (Op::SYM)
+    for (int i = tid; i <= N / 2; i += TH) gx[i] = __ldg(gtab_of(p, b) + i);
+  grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
+  if (flow_stopped(p, blockIdx.y)) return;
   const int cc = tid % C;
   const int jx = (tid / C) % M1, j2 = tid / (M1 * C);  // first / last phase
   const bool has_io = j2 < YB;
   const int ka = (tid / C) % 16, kb = tid / (C * 16);  // operator phase: k1x, k2
-  load_twiddles<N, T>(p, tw);
-  if constexpr (Op::SYM)
-    for (int i = tid; i <= N / 2; i += TH) gx[i] = __ldg(reinterpret_cast<const double2 *>(gtab_of(p, b)) + i);
   double acc[Op::NR > 0 ? Op::NR : 1];
   acc_init<Op::NR, Op::MAXM>(acc);
   __syncthreads();
