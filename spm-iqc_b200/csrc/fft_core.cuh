@@ -33,6 +33,11 @@ constexpr int kCols = 16;       // y-lines (spectral columns) per CTA, plane ker
 // per-CTA global areas that stay resident in L2.
 constexpr int kXgFwd = 1, kXgInv = 2;
 constexpr int kXgRegions = 4;   // exchange-area regions: two per exchange
+// Columns per run of the tile passes' scratch array: a run is what a plane pass
+// reads or writes at once, and a pencil tile takes 32 bytes of each. 256^3 FP64
+// with runs of 2 / 4 / 8 values: joint plane pass 110 / 101 / 99 us, gradient pencil
+// 127 / 133 / 150 us, step 231 / 228 / 243 us.
+constexpr int kRun = 4;
 constexpr int kMaxBatch = 16;   // fields per launch
 constexpr int kScal = 16;       // scalars per field in the scalar block
 constexpr int kRedMax = 8;      // reduction slots per field and CTA
@@ -243,11 +248,20 @@ template <int NR, unsigned MAXM> __device__ __forceinline__ void facc_fold(doubl
   for (int r = 0; r < NR; r++) acc[r] = ((MAXM >> r) & 1u) ? fmax(acc[r], (double)a[r]) : acc[r] + (double)a[r];
 }
 
-// Deterministic block reduction (fixed butterfly + fixed warp order).
-// The result is valid in thread 0. scratch: 32 * NR doubles of shared memory.
-template <int NR, unsigned MAXM>
-__device__ __forceinline__ void block_reduce(double (&a)[NR], double *scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Barrier of n threads of a block (id 1 to 15; n a multiple of 32).
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+// Barrier of the nth threads of group g of a block of G groups (G = 1: the block).
+template <int G> __device__ __forceinline__ void group_sync(int g, int nth) {
+  if constexpr (G > 1) bar_sync(1 + g, nth);
+  else __syncthreads();
+}
+
+// Deterministic reduction over the nth threads of a group (fixed butterfly +
+// fixed warp order). The result is valid in thread 0 of the group. scratch: 32 *
+// NR doubles of shared memory.
+template <int NR, unsigned MAXM, int G = 1>
+__device__ __forceinline__ void block_reduce(double (&a)[NR], double *scratch, int g, int tid, int nth) {
+  const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     double b[NR];
@@ -255,13 +269,13 @@ __device__ __forceinline__ void block_reduce(double (&a)[NR], double *scratch) {
     for (int r = 0; r < NR; r++) b[r] = __shfl_xor_sync(0xffffffffu, a[r], off);
     combine<NR, MAXM>(a, b);
   }
-  __syncthreads();
+  group_sync<G>(g, nth);
   if (lane == 0)
 #pragma unroll
     for (int r = 0; r < NR; r++) scratch[warp * NR + r] = a[r];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
+  group_sync<G>(g, nth);
+  if (tid == 0) {
+    const int nw = nth >> 5;
     for (int w = 1; w < nw; w++) {
       double b[NR];
 #pragma unroll
@@ -271,41 +285,47 @@ __device__ __forceinline__ void block_reduce(double (&a)[NR], double *scratch) {
   }
 }
 
-// Grid reduction: every CTA writes its block total to partials[bidx]; the CTA
-// that finishes last sums all partials in fixed index order (so the result does
-// not depend on scheduling) and returns true in its thread 0 with tot filled.
-template <int NR, unsigned MAXM>
-__device__ __forceinline__ bool grid_reduce(double (&acc)[NR], double *scratch, double *partials,
-                                            unsigned *ticket, int nblk, int bidx, double (&tot)[NR]) {
-  __shared__ int s_last;
-  block_reduce<NR, MAXM>(acc, scratch);
-  if (threadIdx.x == 0) {
+// Grid reduction: every group writes its total to partials[bidx]; the group
+// that finishes last sums all nblk partials in fixed index order (so the result
+// does not depend on scheduling) and returns true in its thread 0 with tot filled.
+template <int NR, unsigned MAXM, int G>
+__device__ __forceinline__ bool group_reduce(double (&acc)[NR], double *scratch, double *partials, unsigned *ticket,
+                                             int nblk, int bidx, int g, int tid, int nth, double (&tot)[NR]) {
+  __shared__ int s_last[G];
+  block_reduce<NR, MAXM, G>(acc, scratch, g, tid, nth);
+  if (tid == 0) {
 #pragma unroll
     for (int r = 0; r < NR; r++) partials[(size_t)bidx * kRedMax + r] = acc[r];
     __threadfence();
     unsigned prev = atomicAdd(ticket, 1u);
-    s_last = (prev == (unsigned)nblk - 1u);
+    s_last[g] = (prev == (unsigned)nblk - 1u);
   }
-  __syncthreads();
-  if (!s_last) return false;
+  group_sync<G>(g, nth);
+  if (!s_last[g]) return false;
   __threadfence();
   double a[NR];
 #pragma unroll
   for (int r = 0; r < NR; r++) a[r] = ((MAXM >> r) & 1u) ? -1.0e308 : 0.0;
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
+  for (int i = tid; i < nblk; i += nth) {
     double b[NR];
 #pragma unroll
     for (int r = 0; r < NR; r++) b[r] = __ldcg(&partials[(size_t)i * kRedMax + r]);
     combine<NR, MAXM>(a, b);
   }
-  block_reduce<NR, MAXM>(a, scratch);
-  if (threadIdx.x == 0) {
+  block_reduce<NR, MAXM, G>(a, scratch, g, tid, nth);
+  if (tid == 0) {
 #pragma unroll
     for (int r = 0; r < NR; r++) tot[r] = a[r];
     *ticket = 0u;
     return true;
   }
   return false;
+}
+// The same over the blocks of a grid.
+template <int NR, unsigned MAXM>
+__device__ __forceinline__ bool grid_reduce(double (&acc)[NR], double *scratch, double *partials,
+                                            unsigned *ticket, int nblk, int bidx, double (&tot)[NR]) {
+  return group_reduce<NR, MAXM, 1>(acc, scratch, partials, ticket, nblk, bidx, 0, threadIdx.x, blockDim.x, tot);
 }
 
 // ------------------------------------------------------------------ async copies
@@ -472,6 +492,14 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
       "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
+                                            uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+      : "memory");
+}
 constexpr long kSpinLimit = 4L << 20;  // polls of ~256 ns: about 1 s
 // Returns false (and sets *err) when the phase did not complete within
 // `limit` polls.
@@ -535,6 +563,13 @@ struct KParams {
   double *statss[kMaxBatch];
 };
 
+// Parameters of the tile passes whose blocks have groups: maps over the
+// scratch p.in for their tensor copies.
+struct KParamsT : KParams {
+  CUtensorMap tm[kMaxBatch];
+};
+template <int G> using TileParams = std::conditional_t<(G > 1), KParamsT, KParams>;
+
 // Parameters of the cluster passes (fft_kernels.cuh).
 struct KParamsC : KParams {
   // Tensor maps of the strided inputs: tmi[b] over p.in[b], tms[b] over p.st[b]
@@ -565,6 +600,10 @@ __device__ __forceinline__ bool flow_stopped(const KParams &p, int b) {
 __device__ __forceinline__ bool flow_pending(const KParams &p, int b) {
   const int *f = flow_of(p, b);
   return f != nullptr && *((volatile const int *)f + FW_PENDING) != 0;
+}
+
+__device__ __forceinline__ void report_error(const KParams &p, int s_err) {
+  if (s_err && p.err && threadIdx.x == 0) atomicExch(p.err, 1);
 }
 
 // Pair kernel G(k^2) (Initialization.cpp:150-166) of a wave vector from the

@@ -118,10 +118,6 @@ template <int N, class T, int RW = kRows, int R = 2> struct XgAreas {
   }
 };
 
-__device__ __forceinline__ void report_error(const KParams &p, int s_err) {
-  if (s_err && p.err && threadIdx.x == 0) atomicExch(p.err, 1);
-}
-
 // --------------------------------------------------------------- plane phases
 // The line-transform phases of the plane passes, shared by plane_fwd,
 // plane_inv and the fused plane_inv_fwd. A CTA of a cluster owns RW z-rows

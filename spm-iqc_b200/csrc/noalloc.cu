@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kNoAllocThreads)
   double a[1] = {0.0};
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     a[0] += (double)__ldg(pb + i) * (double)__ldg(qb + i);
-  spm::block_reduce<1, 0u>(a, red);
+  spm::block_reduce<1, 0u>(a, red, 0, threadIdx.x, blockDim.x);
   if (threadIdx.x == 0) {
     partials[blockIdx.x] = a[0];
     __threadfence();
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kNoAllocThreads)
   __threadfence();
   double t[1] = {0.0};
   for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t[0] += __ldcg(partials + i);
-  spm::block_reduce<1, 0u>(t, red);
+  spm::block_reduce<1, 0u>(t, red, 0, threadIdx.x, blockDim.x);
   if (threadIdx.x == 0) out[b] = t[0] * inv_n;
 }
 

@@ -21,9 +21,8 @@ namespace spm {
 // of the batched ones up to 96^3) are launched that way in any case, and let the next
 // launch in as soon as they run: its blocks are then placed, with their
 // twiddles loaded, when this one completes.
-template <class Tag, class K>
-static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles, const KParams &p0, int nb,
-                        const char *what) {
+template <class Tag, class K, class P>
+static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles, P &p, int nb, const char *what) {
   cudaError_t e = prepare<Tag>(kern, smem, c->device);
   if (e != cudaSuccess) return spm_fail_cuda(e, what);
   static std::atomic<int> resident[32] = {};
@@ -39,7 +38,6 @@ static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles,
     resident[dev].store(most, std::memory_order_relaxed);
   }
   const int nbk = std::min({most, tiles, kPartStride});
-  KParams p = p0;
   p.trigger = 2 * nbk * nb <= most;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nbk, nb, 1);
@@ -56,23 +54,31 @@ static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles,
   return e == cudaSuccess ? 0 : spm_fail_cuda(e, what);
 }
 
-template <int N, class T, class Pro> static int plane_fwd(spm_ctx *c, const KParams &p, int nb) {
+template <int N, class T, class Pro> static int plane_fwd(spm_ctx *c, KParams &p, int nb) {
   struct Tag {};
-  using PG = PlaneGeo<N, T>;
-  return launch_tiles<Tag>(c, plane_fwd_kernel<N, T, Pro>, PG::TH, plane_smem<N, T>(), PG::TILES, p, nb, "plane_fwd");
+  return launch_tiles<Tag>(c, plane_fwd_kernel<N, T, Pro>, N, plane_smem<N, T>(), PlaneGeo<N, T>::TILES, p, nb,
+                           "plane_fwd");
+}
+// The plane kernels that read the scratch: G groups of N threads per block, with
+// the maps of their tensor copies for G > 1.
+template <class Tag, int N, class T, class K> static int launch_inv(spm_ctx *c, K kern, const KParams &p, int nb,
+                                                                    const char *what) {
+  constexpr int G = inv_groups<N, T>();
+  TileParams<G> q;
+  static_cast<KParams &>(q) = p;
+  if constexpr (G > 1)
+    for (int b = 0; b < nb; b++) SPM_TRY(spm_scratch_map(c, p.in[b], &q.tm[b]));
+  return launch_tiles<Tag>(c, kern, G * N, plane_smem<N, T, G>(), PlaneGeo<N, T>::TILES / G, q, nb, what);
 }
 template <int N, class T, class Epi> static int plane_inv(spm_ctx *c, const KParams &p, int nb) {
   struct Tag {};
-  using PG = PlaneGeo<N, T>;
-  return launch_tiles<Tag>(c, plane_inv_kernel<N, T, Epi>, PG::TH, plane_smem<N, T>(), PG::TILES, p, nb, "plane_inv");
+  return launch_inv<Tag, N, T>(c, plane_inv_kernel<N, T, Epi>, p, nb, "plane_inv");
 }
 template <int N, class T, class Epi, class Pro> static int plane_inv_fwd(spm_ctx *c, const KParams &p, int nb) {
   struct Tag {};
-  using PG = PlaneGeo<N, T>;
-  return launch_tiles<Tag>(c, plane_inv_fwd_kernel<N, T, Epi, Pro>, PG::TH, plane_smem<N, T>(), PG::TILES, p, nb,
-                           "plane_inv_fwd");
+  return launch_inv<Tag, N, T>(c, plane_inv_fwd_kernel<N, T, Epi, Pro>, p, nb, "plane_inv_fwd");
 }
-template <int N, class T, class Op> static int pencil(spm_ctx *c, const KParams &p, int nb) {
+template <int N, class T, class Op> static int pencil(spm_ctx *c, KParams &p, int nb) {
   struct Tag {};
   using PG = PencilGeo<N, T>;
   if constexpr (Op::SI)

@@ -193,6 +193,32 @@ int spm_tensor_map(spm_ctx *c, const void *ptr, int kind, CUtensorMap *out) {
   return SPM_OK;
 }
 
+int spm_scratch_map(spm_ctx *c, const void *ptr, CUtensorMap *out) {
+  for (size_t i = c->tmaps.size(); i-- > 0;)
+    if (c->tmaps[i].ptr == ptr && c->tmaps[i].kind == TM_TILE_PLANE) {
+      *out = c->tmaps[i].map;
+      return SPM_OK;
+    }
+  auto fn = encode_fn();
+  if (!fn) return spm_fail(SPM_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  const cuuint64_t N = (cuuint64_t)c->N, YB = N / 32, MR = N / 2 / kRun, run = 16 * kRun;  // bytes of a run
+  const cuuint64_t dims[4] = {2 * kRun, YB * N, MR, 32};
+  const cuuint64_t strides[3] = {run, run * YB * N, run * YB * N * MR};
+  const cuuint32_t box[4] = {2 * kRun, 1, (cuuint32_t)MR, 32};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  TmEntry e;
+  e.ptr = ptr;
+  e.kind = TM_TILE_PLANE;
+  const CUresult r = fn(&e.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void *>(ptr), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return spm_fail(SPM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  if (c->tmaps.size() >= 64) c->tmaps.erase(c->tmaps.begin());
+  c->tmaps.push_back(e);
+  *out = e.map;
+  return SPM_OK;
+}
+
 // Reads (and clears) the error word that bounded waits set on timeout.
 int spm_check_device_error(spm_ctx *c) {
   int err = 0;

@@ -14,7 +14,8 @@
 enum TmKind {
   TM_PENCIL = 0,     // 8 complex columns x 1 ky row x all N x
   TM_PLANE_INV = 1,  // 16 complex columns x all N ky x 1 x-plane
-  TM_PENCIL4 = 2     // 4 complex columns x 1 ky row x all N x (narrow pencil tiles)
+  TM_PENCIL4 = 2,    // 4 complex columns x 1 ky row x all N x (narrow pencil tiles)
+  TM_TILE_PLANE = 3  // a plane tile of a tile-pass scratch: every k1 and column of one (j2, x)
 };
 struct TmEntry {
   const void *ptr;
@@ -84,6 +85,9 @@ int spm_flow_init(spm_ctx *c, cudaStream_t s);    // go = 1, iter = 0
 int spm_ensure_stats(spm_ctx *c, int n);          // per-step record capacity
 // Tensor map of kind `kind` over the packed spectrum at ptr (cached per context).
 int spm_tensor_map(spm_ctx *c, const void *ptr, int kind, CUtensorMap *out);
+// The map TM_TILE_PLANE over an FP64 scratch array of the tile passes,
+// [k1][column / 4][j2 N + x][2 * 4 reals].
+int spm_scratch_map(spm_ctx *c, const void *ptr, CUtensorMap *out);
 void spm_free_extra(spm_ctx *c);
 // Creates (once) the FP32 twin context and its two FP32 fields, and binds it
 // to the context's stream, cancel flag and tuning.

@@ -46,12 +46,6 @@ template <int N> struct Geo {
 // and 160^3; at 256^3 one block of 512 threads per SM instead of two of 256.)
 template <class T> constexpr int tile_cols() { return (int)(32 / sizeof(c2<T>)); }
 
-// Columns per run of the scratch array: a run is what a plane pass reads or
-// writes at once, and a pencil tile takes 32 bytes of each. 256^3 FP64 with runs
-// of 2 / 4 / 8 values: plane pass 132 / 114 / 106 us, gradient pencil 138 / 145 /
-// 163 us.
-constexpr int kRun = 4;
-
 // Position of (k1, column, j2, x) in the scratch array.
 template <int N, int R = kRun>
 __device__ __forceinline__ size_t scratch_index(int k1, int col, int j2, int x) {
@@ -68,18 +62,32 @@ template <int N, class T> __device__ __forceinline__ size_t state_kx_stride(int 
   return tiled ? (size_t)tile_cols<T>() : (size_t)N * Geo<N>::M;
 }
 
+// Groups per block of the plane passes that read the scratch (plane_inv,
+// plane_inv_fwd) at 256^3 FP64: a block of 512 threads (one per SM) is two
+// groups of N threads that work on tiles of their own with barriers of their
+// own, and share one 64 KB stage in shared memory into which the next tile is
+// copied (one tensor copy) while the groups compute. Two blocks of one group each
+// with loads into registers (every tile waits for its loads): 113 against
+// 101 us for the joint pass. Smaller grids run as fast without (their
+// scratch stays in L2), and so does plane_fwd (contiguous rows); the pencil pass
+// was slower staged (141 against 132 us: 32-byte rows, and the stage leaves
+// the L1 too small for the state's loads).
+template <int N, class T> constexpr int inv_groups() { return sizeof(T) == 8 && N == 256 ? 2 : 1; }
+
 // Plane pass: N threads per tile of 32 rows x M complex values (16 per
 // thread), rows padded by one value. 512 threads per SM in FP64 (up to 128
-// registers each), 1024 in FP32.
-template <int N, class T> struct PlaneGeo {
-  static constexpr int TH = N;
+// registers each), 1024 in FP32. G: groups per block (inv_groups).
+template <int N, class T, int GR = 1> struct PlaneGeo {
+  static constexpr int TH = N, G = GR;
+  static constexpr int STAGE = G > 1 ? kRows * Geo<N>::M : 0;
   static constexpr int RS = Geo<N>::M + 1;  // row stride
   static constexpr int UNITS = kRows * RS;
   static constexpr int TILES = N * Geo<N>::YB;  // per field
-  static constexpr int CPS = (sizeof(T) == 8 ? 512 : 1024) / N;
+  static constexpr int CPS = (sizeof(T) == 8 ? 512 : 1024) / (G * N);
 };
-template <int N, class T> constexpr size_t plane_smem() {
-  return sizeof(c2<T>) * (N + PlaneGeo<N, T>::UNITS) + sizeof(double) * 32 * kRedMax + 16;
+template <int N, class T, int G = 1> constexpr size_t plane_smem() {
+  using PG = PlaneGeo<N, T, G>;
+  return sizeof(c2<T>) * (N + PG::STAGE + G * PG::UNITS) + G * sizeof(double) * 32 * kRedMax + (G > 1 ? 16 * G + 128 : 0);
 }
 
 // Pencil pass: 16 YB C threads per tile of N x YB x C complex values; the
@@ -98,8 +106,42 @@ template <int N, class T> struct PencilGeo {
 };
 template <int N, class T> constexpr size_t pencil_smem() {
   return sizeof(c2<T>) * (N + PencilGeo<N, T>::UNITS) + sizeof(double2) * (N / 2 + 1) +
-         sizeof(double) * 32 * kRedMax + 16;
+         sizeof(double) * 32 * kRedMax;
 }
+
+// The stage shared by a block's G groups: group g has a "full" barrier
+// (completed by the copy's bytes) and an "empty" one (an arrival per warp of the
+// group that has read its tile). The copy of the block's tile i + 1 is issued
+// by the group of tile i once that group has read its own.
+template <int N, int G> struct Stage {
+  uint64_t *full, *empty;  // [G]
+  int *err;
+  __device__ void init(uint64_t *bars, int *s_err) {
+    full = bars;
+    empty = bars + G;
+    err = s_err;
+    if (threadIdx.x == 0) {
+      for (int g = 0; g < G; g++) {
+        mbar_init(full + g, 1);
+        mbar_init(empty + g, N / 32);
+      }
+      *s_err = 0;
+      fence_barrier_init();
+    }
+  }
+  // The group's tile of round `round` has arrived.
+  __device__ void wait(int g, int round) { mbar_wait(full + g, round & 1, err); }
+  // This warp has read it; thread 0 of the group then issues the next copy.
+  template <class F> __device__ void next(int g, int tid, int round, F issue) {
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(empty + g);
+    if (tid == 0) {
+      mbar_wait(empty + g, round & 1, err);
+      fence_proxy_async();
+      issue((g + 1) % G);
+    }
+  }
+};
 
 // --------------------------------------------------------------- plane phases
 // One tile in three phases per direction, each on registers with one exchange
@@ -153,17 +195,18 @@ template <int N, class T> struct Plane {
     }
   }
 
-  // scratch -> y: the inverse of y_fwd (unnormalised).
-  __device__ static void y_inv(T2 *buf, const T2 *tw, int tid, const T2 *src, int x, int j2) {
+  // scratch -> y: the inverse of y_fwd (unnormalised). o: the values k1 = 8 b,
+  // 8 b + 1, ... of column q, kst apart (in the scratch or the stage); read()
+  // is called when they have been loaded.
+  template <class F> __device__ static void y_inv(T2 *buf, const T2 *tw, int tid, const T2 *o, size_t kst, F read) {
     const int b = (tid >> 4) & 1, q = (tid >> 5) * 16 + (tid & 15);
-    const T2 *o = src + scratch_index<N>(8 * b, q, j2, x);
-    constexpr size_t KST = (size_t)M * YB * N;
     T2 lo[8], v[16];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-      lo[i] = o[i * KST];
-      v[i] = o[(i + 16) * KST];
+      lo[i] = o[i * kst];
+      v[i] = o[(i + 16) * kst];
     }
+    read();
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const T2 s = cadd(lo[i], v[i]);
@@ -285,6 +328,80 @@ template <int N, class T> struct Plane {
   }
 };
 
+// A plane kernel's loop over the tiles of this thread's group: tiles vb + i G
+// gridDim.x, vb = blockIdx.x + g gridDim.x (what a grid of G gridDim.x one-group
+// blocks does, so that the sums are the same). With INV the tile's input comes
+// through the stage (or straight from the scratch, G = 1), and body(x, j2)
+// follows the inverse class phase.
+template <int N, class T, bool INV, int G> struct PlaneLoop {
+  using T2 = c2<T>;
+  using PG = PlaneGeo<N, T, G>;
+  using P = Plane<N, T>;
+  T2 *tw, *buf, *stage;
+  double *red;
+  int g, tid;
+  Stage<N, G> st;
+  __device__ PlaneLoop(unsigned char *raw, int *s_err) {
+    stage = reinterpret_cast<T2 *>(G > 1 ? smem_base128(raw) : raw);
+    tw = stage + PG::STAGE;
+    T2 *work = tw + N;
+    double *reds = reinterpret_cast<double *>(work + G * PG::UNITS);
+    g = G > 1 ? threadIdx.x / N : 0;
+    tid = G > 1 ? threadIdx.x % N : threadIdx.x;
+    buf = work + g * PG::UNITS;
+    red = reds + g * 32 * kRedMax;
+    if constexpr (G > 1) st.init(reinterpret_cast<uint64_t *>(reds + G * 32 * kRedMax), s_err);
+  }
+  // barrier of the threads that share a tile
+  __device__ void sync() const {
+    if constexpr (G > 1) bar_sync(1 + g, N);
+    else __syncthreads();
+  }
+  template <class F> __device__ void run(const TileParams<G> &p, int b, F body) {
+    const T2 *src = reinterpret_cast<const T2 *>(p.in[b]);
+    auto issue = [&](int tile, int gg) {
+      if constexpr (G > 1) {
+        if (tile >= PG::TILES) return;
+        mbar_expect_tx(st.full + gg, (unsigned)(PG::STAGE * sizeof(T2)));
+        tma_load_4d(stage, &p.tm[b], 0, (tile % P::YB) * N + tile / P::YB, 0, 0, st.full + gg);
+      }
+    };
+    if constexpr (G > 1)
+      if (threadIdx.x == 0) issue(blockIdx.x, 0);
+    int round = 0;
+    for (int tile = blockIdx.x + g * gridDim.x; tile < PG::TILES; tile += G * gridDim.x, round++) {
+      const int x = tile / P::YB, j2 = tile % P::YB;
+      if constexpr (INV) {
+        const int kb = 8 * ((tid >> 4) & 1), q = (tid >> 5) * 16 + (tid & 15);
+        if constexpr (G > 1) {
+          st.wait(g, round);
+          P::y_inv(buf, tw, tid, stage + kb * P::M + q, P::M,
+                   [&]() { st.next(g, tid, round, [&](int gg) { issue(tile + gridDim.x, gg); }); });
+        } else {
+          P::y_inv(buf, tw, tid, src + scratch_index<N>(kb, q, j2, x), (size_t)P::M * P::YB * N, []() {});
+        }
+        sync();
+        P::class_inv(buf, tw, tid);
+        sync();
+      }
+      body(x, j2);
+    }
+    if constexpr (G > 1) {  // a wait ran out
+      __syncthreads();
+      report_error(p, *st.err);
+    }
+  }
+  // Grid reduction over the threads of every group (grid_reduce); fin(tot) runs
+  // in one thread.
+  template <int NR, unsigned MAXM, class F>
+  __device__ void reduce(const KParams &p, int b, double (&acc)[NR], F fin) {
+    double tot[NR];
+    if (group_reduce<NR, MAXM, G>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax, p.tickets + b,
+                                  G * gridDim.x, blockIdx.x + g * gridDim.x, g, tid, G > 1 ? N : blockDim.x, tot))
+      fin(tot);
+  }
+};
+
 template <int N, class T> __device__ __forceinline__ void load_twiddles(const KParams &p, c2<T> *tw) {
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = reinterpret_cast<const c2<T> *>(p.tw)[i];
 }
@@ -309,27 +426,26 @@ __device__ __forceinline__ void run_prologue(F &&points, ACC &acc) {
 //        (x = reals idx, idx+1 of the input field; returns the values to transform)
 //      __device__ static void fin(const KParams&, int b, const double (&tot)[NR]);
 template <int N, class T, class Pro>
-__global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
+__global__ void __launch_bounds__(N, PlaneGeo<N, T>::CPS)
     plane_fwd_kernel(const __grid_constant__ KParams p) {
   using T2 = c2<T>;
   using P = Plane<N, T>;
-  using PG = PlaneGeo<N, T>;
   constexpr int N1 = P::N1, YB = P::YB;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  T2 *tw = reinterpret_cast<T2 *>(smem_raw);
-  T2 *buf = tw + N;
-  double *red = reinterpret_cast<double *>(buf + PG::UNITS + (PG::UNITS & 1));
+  __shared__ int s_err;
+  PlaneLoop<N, T, false, 1> loop(smem_raw, &s_err);
+  T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
-  const int tid = threadIdx.x, b = blockIdx.y;
+  const int tid = loop.tid, b = blockIdx.y;
   const T *src = reinterpret_cast<const T *>(p.in[b]);
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
   double acc[Pro::NR > 0 ? Pro::NR : 1];
   acc_init<Pro::NR, Pro::MAXM>(acc);
-  for (int tile = blockIdx.x; tile < PG::TILES; tile += gridDim.x) {
-    const int x = tile / YB, j2 = tile % YB;
+  __syncthreads();
+  loop.run(p, b, [&](int x, int j2) {
     P::rows(tid, [&](int r, int jz) {
       const size_t off = ((size_t)x * N + YB * r + j2) * N;
       const T2 *row = reinterpret_cast<const T2 *>(src + off);
@@ -345,18 +461,14 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
           acc);
       P::row_store_fwd(buf, r, jz, v);
     });
-    __syncthreads();
+    loop.sync();
     P::class_fwd(buf, tw, tid);
-    __syncthreads();
+    loop.sync();
     P::y_fwd(buf, tw, tid, dst, x, j2);
-    __syncthreads();
-  }
-  if constexpr (Pro::NR > 0) {
-    double tot[Pro::NR];
-    if (grid_reduce<Pro::NR, Pro::MAXM>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax,
-                                        p.tickets + b, gridDim.x, blockIdx.x, tot))
-      Pro::fin(p, b, tot);
-  }
+    loop.sync();
+  });
+  if constexpr (Pro::NR > 0)
+    loop.template reduce<Pro::NR, Pro::MAXM>(p, b, acc, [&](double (&tot)[Pro::NR]) { Pro::fin(p, b, tot); });
 }
 
 // --------------------------------------------------------------- plane_inv
@@ -366,32 +478,26 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
 //        (y = unnormalised inverse transform at reals idx, idx+1; returns values to store)
 //      __device__ static void fin(const KParams&, int b, const double (&tot)[NR]);
 template <int N, class T, class Epi>
-__global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
-    plane_inv_kernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_groups<N, T>()>::CPS)
+    plane_inv_kernel(const __grid_constant__ TileParams<inv_groups<N, T>()> p) {
   using T2 = c2<T>;
   using P = Plane<N, T>;
-  using PG = PlaneGeo<N, T>;
+  constexpr int G = inv_groups<N, T>();
   constexpr int N1 = P::N1, YB = P::YB;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  T2 *tw = reinterpret_cast<T2 *>(smem_raw);
-  T2 *buf = tw + N;
-  double *red = reinterpret_cast<double *>(buf + PG::UNITS + (PG::UNITS & 1));
+  __shared__ int s_err;
+  PlaneLoop<N, T, true, G> loop(smem_raw, &s_err);
+  T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
-  const int tid = threadIdx.x, b = blockIdx.y;
-  const T2 *src = reinterpret_cast<const T2 *>(p.in[b]);
+  const int tid = loop.tid, b = blockIdx.y;
   T *outb = reinterpret_cast<T *>(p.out[b]);  // null: reductions only
   double acc[Epi::NR > 0 ? Epi::NR : 1];
   acc_init<Epi::NR, Epi::MAXM>(acc);
   __syncthreads();
-  for (int tile = blockIdx.x; tile < PG::TILES; tile += gridDim.x) {
-    const int x = tile / YB, j2 = tile % YB;
-    P::y_inv(buf, tw, tid, src, x, j2);
-    __syncthreads();
-    P::class_inv(buf, tw, tid);
-    __syncthreads();
+  loop.run(p, b, [&](int x, int j2) {
     P::rows(tid, [&](int r, int jz) {
       const size_t off = ((size_t)x * N + YB * r + j2) * N;
       T2 v[N1];
@@ -406,14 +512,10 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
           },
           acc);
     });
-    __syncthreads();
-  }
-  if constexpr (Epi::NR > 0) {
-    double tot[Epi::NR];
-    if (grid_reduce<Epi::NR, Epi::MAXM>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax,
-                                        p.tickets + b, gridDim.x, blockIdx.x, tot))
-      Epi::fin(p, b, tot);
-  }
+    loop.sync();
+  });
+  if constexpr (Epi::NR > 0)
+    loop.template reduce<Epi::NR, Epi::MAXM>(p, b, acc, [&](double (&tot)[Epi::NR]) { Epi::fin(p, b, tot); });
 }
 
 // --------------------------------------------------------------- plane_inv_fwd
@@ -424,38 +526,32 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
 // (the pencil pass armed FW_PENDING): the forward half is then skipped. A chain
 // of K steps is plane_fwd, K pencils, K-1 of these and one plane_inv.
 template <int N, class T, class Epi, class Pro>
-__global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
-    plane_inv_fwd_kernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_groups<N, T>()>::CPS)
+    plane_inv_fwd_kernel(const __grid_constant__ TileParams<inv_groups<N, T>()> p) {
   using T2 = c2<T>;
   using P = Plane<N, T>;
-  using PG = PlaneGeo<N, T>;
+  constexpr int G = inv_groups<N, T>();
   constexpr int N1 = P::N1, YB = P::YB;
   constexpr int NE = Epi::NR, NP = Pro::NR, NA = (NE + NP > 0) ? NE + NP : 1;
   static_assert(NA <= kRedMax, "reduction count");
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  T2 *tw = reinterpret_cast<T2 *>(smem_raw);
-  T2 *buf = tw + N;
-  double *red = reinterpret_cast<double *>(buf + PG::UNITS + (PG::UNITS & 1));
+  __shared__ int s_err;
+  PlaneLoop<N, T, true, G> loop(smem_raw, &s_err);
+  T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
   // uniform over the grid: set by the pencil pass of this step, before launch
   const bool stop = flow_pending(p, blockIdx.y);
-  const int tid = threadIdx.x, b = blockIdx.y;
-  const T2 *src = reinterpret_cast<const T2 *>(p.in[b]);
+  const int tid = loop.tid, b = blockIdx.y;
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
   T *phi = reinterpret_cast<T *>(p.sto[b]);
   double acc_e[NE > 0 ? NE : 1], acc_p[NP > 0 ? NP : 1];
   acc_init<NE, Epi::MAXM>(acc_e);
   acc_init<NP, Pro::MAXM>(acc_p);
   __syncthreads();
-  for (int tile = blockIdx.x; tile < PG::TILES; tile += gridDim.x) {
-    const int x = tile / YB, j2 = tile % YB;
-    P::y_inv(buf, tw, tid, src, x, j2);
-    __syncthreads();
-    P::class_inv(buf, tw, tid);
-    __syncthreads();
+  loop.run(p, b, [&](int x, int j2) {
     P::rows(tid, [&](int r, int jz) {
       const size_t off = ((size_t)x * N + YB * r + j2) * N;
       T2 v[N1];
@@ -478,32 +574,31 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
           acc_p);
       P::row_store_fwd(buf, r, jz, v);
     });
-    __syncthreads();
+    loop.sync();
     if (!stop) {
       P::class_fwd(buf, tw, tid);
-      __syncthreads();
+      loop.sync();
       P::y_fwd(buf, tw, tid, dst, x, j2);
-      __syncthreads();
+      loop.sync();
     }
-  }
+  });
   if (stop) {  // u back from tile order (p.aux0) into the caller's packed spectrum (p.aux1)
     constexpr int M = Geo<N>::M;
     const T2 *ut = reinterpret_cast<const T2 *>(p.aux0[b]);
     T2 *u = reinterpret_cast<T2 *>(const_cast<void *>(p.aux1[b]));
     for (int row = blockIdx.x; row < N * N; row += gridDim.x) {
       const int kx = row / N, ky = row % N;
-      for (int c = tid; c < M; c += PG::TH)
+      for (int c = threadIdx.x; c < M; c += blockDim.x)
         u[(size_t)row * M + c] = ut[state_index<N, T>(ky % 32, ky / 32, kx, c, 1)];
     }
   }
-  double all[NA], tot[NA];
+  double all[NA];
 #pragma unroll
   for (int r = 0; r < NE; r++) all[r] = acc_e[r];
 #pragma unroll
   for (int r = 0; r < NP; r++) all[NE + r] = acc_p[r];
   if constexpr (NE + NP == 0) all[0] = 0.0;
-  if (grid_reduce<NA, (Epi::MAXM | (Pro::MAXM << NE))>(all, red, p.partials + (size_t)b * kPartStride * kRedMax,
-                                                        p.tickets + b, gridDim.x, blockIdx.x, tot)) {
+  loop.template reduce<NA, (Epi::MAXM | (Pro::MAXM << NE))>(p, b, all, [&](double (&tot)[NA]) {
     double te[NE > 0 ? NE : 1], tp[NP > 0 ? NP : 1];
 #pragma unroll
     for (int r = 0; r < NE; r++) te[r] = tot[r];
@@ -511,7 +606,7 @@ __global__ void __launch_bounds__(PlaneGeo<N, T>::TH, PlaneGeo<N, T>::CPS)
     for (int r = 0; r < NP; r++) tp[r] = tot[NE + r];
     Epi::fin(p, b, te);
     if (!stop) Pro::fin(p, b, tp);
-  }
+  });
 }
 
 // --------------------------------------------------------------- pencil
