@@ -55,6 +55,7 @@ template <class T> struct ProGrad {
 // and sum((-Tau - 2 Gamma phi + 3 phi^2) v) so the epilogue can remove the mean
 // mu = G(0) mean(v) + mean(c(phi) v) without a second pass (aux0 = phi).
 template <class T> struct ProHv {
+  static constexpr int AUX = 1;
   static constexpr int NR = 2;
   static constexpr unsigned MAXM = 0;
   __device__ static c2<T> pro(const KParams &p, int b, size_t idx, c2<T> x, double (&acc)[2]) {
@@ -109,6 +110,7 @@ template <class T> struct ProPrecond {
 // FACC: in FP32 the four sums run in FP32 over a row's points of one thread
 // before they join the FP64 totals.
 template <class T> struct ProForce {
+  static constexpr int AUX = 2;
   static constexpr int NR = 4;
   static constexpr unsigned MAXM = 0;
   static constexpr bool FACC = true;
@@ -134,6 +136,7 @@ template <class T> struct ProForce {
 // SPM tangent (SPM.cpp:15-32): transform d = Phi1 - Phi0 (in = Phi1, aux0 =
 // Phi0) and accumulate |d|^2; the pencil scales by 1/||d||.
 template <class T> struct ProTangent {
+  static constexpr int AUX = 1;
   static constexpr int NR = 1;
   static constexpr unsigned MAXM = 0;
   static constexpr bool FACC = true;
@@ -152,6 +155,7 @@ template <class T> struct ProTangent {
 // with N = Tau x + Gamma x^2 - x^3 (its mean only reaches the k = 0 mode,
 // which the step zeroes) and T = 2 PV(f) (aux0); beta in m.factor.
 template <class T> struct ProHisd {
+  static constexpr int AUX = 1;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
   __device__ static c2<T> pro(const KParams &p, int b, size_t idx, c2<T> x, double (&)[1]) {
@@ -381,6 +385,7 @@ template <class T> struct EpiFlow {
 // minus its mean (= -mean f), negated. Also sums the result squared
 // (nrmp, BasicOperators.cpp:158-164). aux0 = phi.
 template <class T> struct EpiNgrad {
+  static constexpr int AUX = 1;
   static constexpr int NR = 1;
   static constexpr unsigned MAXM = 0;
   static constexpr bool FACC = true;
@@ -407,6 +412,7 @@ template <class T> struct EpiNgrad {
 // scal[SC_SUM2] = mean(v), so the caller can apply the projection where it uses
 // the product (no pass over phi before the transform). aux0 = phi, aux1 = v.
 template <class T> struct EpiHvRaw {
+  static constexpr int AUX = 2;
   static constexpr int NR = 3;
   static constexpr unsigned MAXM = 0;
   __device__ static c2<T> epi(const KParams &p, int b, size_t idx, c2<T> y, double (&acc)[3]) {
@@ -429,6 +435,7 @@ template <class T> struct EpiHvRaw {
 };
 
 template <class T> struct EpiHv {
+  static constexpr int AUX = 2;
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
   __device__ static c2<T> epi(const KParams &p, int b, size_t idx, c2<T> y, double (&)[1]) {

@@ -40,7 +40,7 @@ static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles,
   const int nbk = std::min({most, tiles, kPartStride});
   p.trigger = 2 * nbk * nb <= most;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nbk, nb, 1);
+  cfg.gridDim = dim3(nb, nbk, 1);
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = c->stream;

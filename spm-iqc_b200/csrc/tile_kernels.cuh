@@ -143,6 +143,14 @@ template <int N, int G> struct Stage {
   }
 };
 
+// The fields of a launch share its grid field-fastest: the blocks that work on
+// the same tiles of the fields of a block run together, so that what the fields
+// share (phi of Hessian products, the tangent of force steps) is read from
+// memory once. Which tiles a block takes does not depend on the number of fields.
+__device__ __forceinline__ int field_id() { return blockIdx.x; }
+__device__ __forceinline__ int block_id() { return blockIdx.y; }
+__device__ __forceinline__ int block_count() { return gridDim.y; }
+
 // --------------------------------------------------------------- plane phases
 // One tile in three phases per direction, each on registers with one exchange
 // through `buf` in between (row r = j1, RS values apart):
@@ -328,8 +336,22 @@ template <int N, class T> struct Plane {
   }
 };
 
+// Field arrays a policy reads beside its input (p.aux0, p.aux1): X::AUX, else none.
+template <class X, class = void> struct AuxOf : std::integral_constant<int, 0> {};
+template <class X> struct AuxOf<X, std::void_t<decltype(X::AUX)>> : std::integral_constant<int, X::AUX> {};
+
+// Asks for the 32 rows of tile (x, j2) of a real field to be brought into L2 (one
+// warp; bulk prefetches want 16-byte alignment, which FP32 fields need not have).
+// From 96^3 to 192^3 only (Hessian products in blocks of 8, FP64, without and
+// with: 96^3 19.8 / 19.0, 128^3 38 / 35, 160^3 78 / 75, 192^3 151 / 136 us each;
+// but 64^3 6.8 / 7.2 and 256^3 278 / 281 us, one product 320 / 335).
+template <int N, class T> __device__ __forceinline__ void prefetch_rows(const void *field, int tid, int x, int j2) {
+  if (N >= 96 && N <= 192 && ((uintptr_t)field & 15u) == 0 && field && tid < kRows)
+    prefetch_l2(reinterpret_cast<const T *>(field) + ((size_t)x * N + Geo<N>::YB * tid + j2) * N, N * sizeof(T));
+}
+
 // A plane kernel's loop over the tiles of this thread's group: tiles vb + i G
-// gridDim.x, vb = blockIdx.x + g gridDim.x (what a grid of G gridDim.x one-group
+// block_count(), vb = block_id() + g block_count() (what a grid of G block_count() one-group
 // blocks does, so that the sums are the same). With INV the tile's input comes
 // through the stage (or straight from the scratch, G = 1), and body(x, j2)
 // follows the inverse class phase.
@@ -357,7 +379,7 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
     if constexpr (G > 1) bar_sync(1 + g, N);
     else __syncthreads();
   }
-  template <class F> __device__ void run(const TileParams<G> &p, int b, F body) {
+  template <int AUX = 0, class F> __device__ void run(const TileParams<G> &p, int b, F body) {
     const T2 *src = reinterpret_cast<const T2 *>(p.in[b]);
     auto issue = [&](int tile, int gg) {
       if constexpr (G > 1) {
@@ -367,16 +389,19 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
       }
     };
     if constexpr (G > 1)
-      if (threadIdx.x == 0) issue(blockIdx.x, 0);
+      if (threadIdx.x == 0) issue(block_id(), 0);
     int round = 0;
-    for (int tile = blockIdx.x + g * gridDim.x; tile < PG::TILES; tile += G * gridDim.x, round++) {
+    for (int tile = block_id() + g * block_count(); tile < PG::TILES; tile += G * block_count(), round++) {
       const int x = tile / P::YB, j2 = tile % P::YB;
       if constexpr (INV) {
         const int kb = 8 * ((tid >> 4) & 1), q = (tid >> 5) * 16 + (tid & 15);
+        // the epilogue's rows towards L2
+        if constexpr (AUX > 0) prefetch_rows<N, T>(p.aux0[b], tid, x, j2);
+        if constexpr (AUX > 1) prefetch_rows<N, T>(p.aux1[b], tid, x, j2);
         if constexpr (G > 1) {
           st.wait(g, round);
           P::y_inv(buf, tw, tid, stage + kb * P::M + q, P::M,
-                   [&]() { st.next(g, tid, round, [&](int gg) { issue(tile + gridDim.x, gg); }); });
+                   [&]() { st.next(g, tid, round, [&](int gg) { issue(tile + block_count(), gg); }); });
         } else {
           P::y_inv(buf, tw, tid, src + scratch_index<N>(kb, q, j2, x), (size_t)P::M * P::YB * N, []() {});
         }
@@ -397,7 +422,7 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
   __device__ void reduce(const KParams &p, int b, double (&acc)[NR], F fin) {
     double tot[NR];
     if (group_reduce<NR, MAXM, G>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax, p.tickets + b,
-                                  G * gridDim.x, blockIdx.x + g * gridDim.x, g, tid, G > 1 ? N : blockDim.x, tot))
+                                  G * block_count(), block_id() + g * block_count(), g, tid, G > 1 ? N : blockDim.x, tot))
       fin(tot);
   }
 };
@@ -438,14 +463,19 @@ __global__ void __launch_bounds__(N, PlaneGeo<N, T>::CPS)
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
-  if (flow_stopped(p, blockIdx.y)) return;
-  const int tid = loop.tid, b = blockIdx.y;
+  if (flow_stopped(p, field_id())) return;
+  const int tid = loop.tid, b = field_id();
   const T *src = reinterpret_cast<const T *>(p.in[b]);
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
   double acc[Pro::NR > 0 ? Pro::NR : 1];
   acc_init<Pro::NR, Pro::MAXM>(acc);
   __syncthreads();
   loop.run(p, b, [&](int x, int j2) {
+    if (const int next = x * YB + j2 + block_count(); next < PlaneGeo<N, T>::TILES) {
+      prefetch_rows<N, T>(src, tid, next / YB, next % YB);
+      if constexpr (AuxOf<Pro>::value > 0) prefetch_rows<N, T>(p.aux0[b], tid, next / YB, next % YB);
+      if constexpr (AuxOf<Pro>::value > 1) prefetch_rows<N, T>(p.aux1[b], tid, next / YB, next % YB);
+    }
     P::rows(tid, [&](int r, int jz) {
       const size_t off = ((size_t)x * N + YB * r + j2) * N;
       const T2 *row = reinterpret_cast<const T2 *>(src + off);
@@ -491,13 +521,13 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
-  if (flow_stopped(p, blockIdx.y)) return;
-  const int tid = loop.tid, b = blockIdx.y;
+  if (flow_stopped(p, field_id())) return;
+  const int tid = loop.tid, b = field_id();
   T *outb = reinterpret_cast<T *>(p.out[b]);  // null: reductions only
   double acc[Epi::NR > 0 ? Epi::NR : 1];
   acc_init<Epi::NR, Epi::MAXM>(acc);
   __syncthreads();
-  loop.run(p, b, [&](int x, int j2) {
+  loop.template run<AuxOf<Epi>::value>(p, b, [&](int x, int j2) {
     P::rows(tid, [&](int r, int jz) {
       const size_t off = ((size_t)x * N + YB * r + j2) * N;
       T2 v[N1];
@@ -541,10 +571,10 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
-  if (flow_stopped(p, blockIdx.y)) return;
+  if (flow_stopped(p, field_id())) return;
   // uniform over the grid: set by the pencil pass of this step, before launch
-  const bool stop = flow_pending(p, blockIdx.y);
-  const int tid = loop.tid, b = blockIdx.y;
+  const bool stop = flow_pending(p, field_id());
+  const int tid = loop.tid, b = field_id();
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
   T *phi = reinterpret_cast<T *>(p.sto[b]);
   double acc_e[NE > 0 ? NE : 1], acc_p[NP > 0 ? NP : 1];
@@ -586,7 +616,7 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
     constexpr int M = Geo<N>::M;
     const T2 *ut = reinterpret_cast<const T2 *>(p.aux0[b]);
     T2 *u = reinterpret_cast<T2 *>(const_cast<void *>(p.aux1[b]));
-    for (int row = blockIdx.x; row < N * N; row += gridDim.x) {
+    for (int row = block_id(); row < N * N; row += block_count()) {
       const int kx = row / N, ky = row % N;
       for (int c = threadIdx.x; c < M; c += blockDim.x)
         u[(size_t)row * M + c] = ut[state_index<N, T>(ky % 32, ky / 32, kx, c, 1)];
@@ -649,13 +679,13 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
   T2 *ex = tw + N;
   double2 *gx = reinterpret_cast<double2 *>(ex + PG::UNITS + (PG::UNITS & 1));  // symbol factors per |K|
   double *red = reinterpret_cast<double *>(gx + N / 2 + 1);
-  const int tid = threadIdx.x, b = blockIdx.y;
+  const int tid = threadIdx.x, b = field_id();
   load_twiddles<N, T>(p, tw);
   if constexpr (Op::SYM)
     for (int i = tid; i <= N / 2; i += TH) gx[i] = __ldg(gtab_of(p, b) + i);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
-  if (flow_stopped(p, blockIdx.y)) return;
+  if (flow_stopped(p, field_id())) return;
   const int cc = tid % C;
   const int jx = (tid / C) % M1, j2 = tid / (M1 * C);  // first / last phase
   const bool has_io = j2 < YB;
@@ -670,8 +700,8 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
 
   // The 16 tiles with the packed column take longer: they go to the first
   // blocks that have one tile less than the others (last round).
-  const int rem = Op::LIN ? 0 : PG::TILES % gridDim.x;
-  for (int v = blockIdx.x; v < PG::TILES; v += gridDim.x) {
+  const int rem = Op::LIN ? 0 : PG::TILES % block_count();
+  for (int v = block_id(); v < PG::TILES; v += block_count()) {
     int g, k1;
     if (v >= rem && v < rem + 16) {
       g = 0;
@@ -846,7 +876,7 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
   if constexpr (Op::NR > 0) {
     double tot[Op::NR];
     if (grid_reduce<Op::NR, Op::MAXM>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax,
-                                      p.tickets + b, gridDim.x, blockIdx.x, tot))
+                                      p.tickets + b, block_count(), block_id(), tot))
       Op::fin(p, b, tot);
   }
 }
