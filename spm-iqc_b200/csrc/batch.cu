@@ -1,13 +1,13 @@
 // Batched gradient flows of independent instances (grids of any supported
-// sizes and parameters): one CUDA graph holds `steps_per_launch` gated steps of
-// every instance, so one graph launch advances all of them. Instances of the
+// sizes and parameters), advanced by rounds of `steps_per_launch` gated steps of
+// every instance. Instances of the
 // same grid size and precision form groups of up to 16 that share every
 // launch (one launch per pass for the whole group, blockIdx.y = instance,
 // each instance with its own model, symbols and flow words); each group runs
-// on its own stream branch, so groups of different sizes overlap on the
+// on its own stream, so groups of different sizes overlap on the
 // device. (With the context knob "batch_group" = 0 on the first instance,
-// every instance gets its own branch and launches instead.) Instances stop
-// on the device (convergence or their step cap); the graph is relaunched until
+// every instance gets its own stream and launches instead.) Instances stop
+// on the device (convergence or their step cap); rounds are launched until
 // every instance has stopped. With switch_tol > 0 the instances first run on
 // their FP32 twins (FP32 transforms, FP64 reductions) to switch_tol, then on
 // FP64 to tol_grad.
@@ -100,44 +100,60 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
     ctx[i]->m.tol_grad = tol;
     ctx[i]->m.max_steps = caps ? caps[i] : max_steps;
   }
-  // one step of every group outside the capture sets up kernel attributes
-  // and tensor maps; it counts as the first step of the flow
-  for (int i = 0; i < n; i++) ctx[i]->stream = s0;
-  for (const auto &grp : groups) SPM_TRY(group_steps(ctx, phi, uh, grp, 1));
+  // K steps of every group, each on its own stream between s0 and s0
+  cudaError_t e = cudaSuccess;
+  int rc = SPM_OK;
+  auto advance = [&]() {
+    e = cudaEventRecord(st.ev[ng], s0);
+    for (int g = 0; g < ng && rc == SPM_OK && e == cudaSuccess; g++) {
+      e = cudaStreamWaitEvent(st.s[g], st.ev[ng], 0);
+      for (int i : groups[g]) ctx[i]->stream = st.s[g];
+      rc = group_steps(ctx, phi, uh, groups[g], K);
+      if (e == cudaSuccess) e = cudaEventRecord(st.ev[g], st.s[g]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(s0, st.ev[g], 0);
+    }
+  };
+  // Up to kDirectGroups groups are launched step by step: two launches a step
+  // and group take the host less time than the device needs for the step, and a
+  // graph costs its capture and instantiation first (2 ms for three groups of
+  // 16 steps, against 85 us a step on the device). Many groups (instances
+  // that share no launch) go through a captured graph of K steps.
+  constexpr int kDirectGroups = 8;
+  const bool direct = ng <= kDirectGroups;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  cudaError_t e = cudaStreamBeginCapture(s0, cudaStreamCaptureModeRelaxed);
-  if (e != cudaSuccess) return spm_fail_cuda(e, "graph capture");
-  e = cudaEventRecord(st.ev[ng], s0);
-  int rc = SPM_OK;
-  for (int g = 0; g < ng && rc == SPM_OK && e == cudaSuccess; g++) {
-    e = cudaStreamWaitEvent(st.s[g], st.ev[ng], 0);
-    for (int i : groups[g]) ctx[i]->stream = st.s[g];
-    rc = group_steps(ctx, phi, uh, groups[g], K);
-    if (e == cudaSuccess) e = cudaEventRecord(st.ev[g], st.s[g]);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s0, st.ev[g], 0);
-  }
-  cudaError_t e2 = cudaStreamEndCapture(s0, &graph);
-  if (rc != SPM_OK) {
-    if (graph) cudaGraphDestroy(graph);
-    return rc;
-  }
-  if (e == cudaSuccess) e = e2;
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-  if (e != cudaSuccess) {
-    if (graph) cudaGraphDestroy(graph);
-    return spm_fail_cuda(e, "graph instantiate");
+  for (int i = 0; i < n; i++) ctx[i]->stream = s0;
+  if (!direct) {
+    // one step of every group outside the capture sets up kernel attributes
+    // and tensor maps; it counts as the first step of the flow
+    for (const auto &grp : groups) SPM_TRY(group_steps(ctx, phi, uh, grp, 1));
+    e = cudaStreamBeginCapture(s0, cudaStreamCaptureModeRelaxed);
+    if (e != cudaSuccess) return spm_fail_cuda(e, "graph capture");
+    advance();
+    cudaError_t e2 = cudaStreamEndCapture(s0, &graph);
+    if (rc != SPM_OK) {
+      if (graph) cudaGraphDestroy(graph);
+      return rc;
+    }
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+    if (e != cudaSuccess) {
+      if (graph) cudaGraphDestroy(graph);
+      return spm_fail_cuda(e, "graph instantiate");
+    }
   }
   std::vector<int> host(8 * (size_t)n);
   std::vector<double> rec;
-  std::vector<int> seen(n, 1);  // the step outside the graph is record 0
+  std::vector<int> seen(n, direct ? 0 : 1);  // (the step outside the graph is record 0)
   std::vector<FloorWatch> watch(n, FloorWatch(tol, stall > 0 ? stall : 1));
   static const int kZero = 0;
   const int launches = (max_steps + K - 1) / K;
   for (int l = 0; l < launches && rc == SPM_OK; l++) {
-    e = cudaGraphLaunch(exec, s0);
+    if (direct) advance();
+    else e = cudaGraphLaunch(exec, s0);
+    if (rc != SPM_OK) break;
     if (e != cudaSuccess) {
-      rc = spm_fail_cuda(e, "graph launch");
+      rc = spm_fail_cuda(e, "batch launch");
       break;
     }
     for (int i = 0; i < n; i++)
@@ -178,8 +194,10 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
     }
     if (all || rc != SPM_OK) break;
   }
-  cudaGraphExecDestroy(exec);
-  cudaGraphDestroy(graph);
+  if (rc != SPM_OK)  // nothing of a failed round stays in flight
+    for (cudaStream_t x : st.s) cudaStreamSynchronize(x);
+  if (exec) cudaGraphExecDestroy(exec);
+  if (graph) cudaGraphDestroy(graph);
   for (int i = 0; i < n; i++) {
     ctx[i]->stream = saved[i];
     ctx[i]->m.tol_grad = 0.0;

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -376,12 +377,15 @@ extern "C" int spm_ctx_create(int N, double L, double Tau, double Gamma, double 
   if (e == cudaSuccess) e = cudaMemset(c->scal, 0, sizeof(double) * kScal * kMaxBatch);
   if (e == cudaSuccess) e = cudaMalloc(&c->flow, sizeof(int) * 8);
   if (e == cudaSuccess) e = cudaMemset(c->flow, 0, sizeof(int) * 8);
-  if (e == cudaSuccess) e = cudaMallocHost(&c->host_scal, sizeof(double) * kScal * kMaxBatch);
-  if (e == cudaSuccess) e = cudaMallocHost(&c->host_flow, sizeof(int) * 8);
+  // one pinned allocation: scalars, step records, flow words
+  if (e == cudaSuccess)
+    e = cudaMallocHost(&c->host_scal, sizeof(double) * (kScal * kMaxBatch + 4 * kHostStats) + sizeof(int) * 8);
   if (e != cudaSuccess) {
     spm_ctx_destroy(c);
     return spm_fail_cuda(e, "context buffers");
   }
+  c->host_stats = c->host_scal + kScal * kMaxBatch;
+  c->host_flow = reinterpret_cast<int *>(c->host_stats + 4 * kHostStats);
   *out = c;
   return SPM_OK;
 }
@@ -406,7 +410,6 @@ extern "C" int spm_ctx_destroy(spm_ctx *c) {
   cudaFree(c->host_phi);
   cudaFree(c->host_uhat);
   if (c->host_scal) cudaFreeHost(c->host_scal);
-  if (c->host_flow) cudaFreeHost(c->host_flow);
   delete c;
   return SPM_OK;
 }
@@ -569,23 +572,42 @@ extern "C" int spm_grad_flow_enqueue(spm_ctx *c, void *phi, void *uhat, int nste
   return rc;
 }
 
-extern "C" int spm_grad_flow_collect(spm_ctx *c, spm_step_stats *stats, int max_records, int *steps_done) {
-  if (!c) return spm_fail(SPM_ERR_ARG, "ctx is NULL");
+// Flow words and the first `ahead` step records (at most kHostStats) into pinned
+// host memory, in one round trip.
+static int read_flow(spm_ctx *c, int ahead) {
   cudaError_t e = cudaMemcpyAsync(c->host_flow, c->flow, sizeof(int) * 8, cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess && ahead > 0)
+    e = cudaMemcpyAsync(c->host_stats, c->stats, sizeof(double) * 4 * (size_t)ahead, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return spm_fail_cuda(e, "grad flow");
-  SPM_TRY(spm_check_device_error(c));
+  return e == cudaSuccess ? SPM_OK : spm_fail_cuda(e, "grad flow");
+}
+
+// The outcome of a flow whose words (and `have` records) read_flow has read.
+static int finish_flow(spm_ctx *c, spm_step_stats *stats, int max_records, int *steps_done, int have) {
+  if (c->host_flow[FW_ERR]) return spm_check_device_error(c);
   const int done = c->host_flow[FW_ITER];
   if (steps_done) *steps_done = done;
   const int n = std::min(done, max_records);
   if (stats && n > 0) {
-    e = cudaMemcpy(stats, c->stats, sizeof(double) * 4 * (size_t)n, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return spm_fail_cuda(e, "stats read");
+    const int h = std::min(n, have);
+    std::memcpy(stats, c->host_stats, sizeof(double) * 4 * (size_t)h);
+    if (h < n) {
+      cudaError_t e = cudaMemcpy(stats + h, c->stats + 4 * (size_t)h, sizeof(double) * 4 * (size_t)(n - h),
+                                 cudaMemcpyDeviceToHost);
+      if (e != cudaSuccess) return spm_fail_cuda(e, "stats read");
+    }
     for (int i = 0; i < n; i++)
       if (!std::isfinite(stats[i].energy) || !std::isfinite(stats[i].grad_norm))
         return spm_fail(SPM_ERR_NONFINITE, "non-finite energy or gradient norm");
   }
   return SPM_OK;
+}
+
+extern "C" int spm_grad_flow_collect(spm_ctx *c, spm_step_stats *stats, int max_records, int *steps_done) {
+  if (!c) return spm_fail(SPM_ERR_ARG, "ctx is NULL");
+  const int have = stats ? std::min(std::min(max_records, c->stats_cap), kHostStats) : 0;
+  SPM_TRY(read_flow(c, have));
+  return finish_flow(c, stats, max_records, steps_done, have);
 }
 
 extern "C" int spm_grad_flow(spm_ctx *c, void *phi, void *uhat, int max_steps, double tol_grad,
@@ -599,23 +621,21 @@ extern "C" int spm_grad_flow(spm_ctx *c, void *phi, void *uhat, int max_steps, d
   flow_init_kernel<<<1, 1, 0, c->stream>>>(c->flow);
   const OpsTable *t = spm_table_of(c);
   c->m.tol_grad = tol_grad;
-  int enq = 0, chunk = 8, rc = SPM_OK;
-  cudaError_t e = cudaSuccess;
+  int enq = 0, chunk = 8, rc = SPM_OK, have = 0;
   while (enq < max_steps) {
     const int n = std::min(chunk, max_steps - enq);
     rc = t->grad_steps(c, phi, uhat, n);
     if (rc != SPM_OK) break;
     enq += n;
-    e = cudaMemcpyAsync(c->host_flow, c->flow, sizeof(int) * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) { rc = spm_fail_cuda(e, "grad flow"); break; }
-    if (c->host_flow[FW_GO] == 0) break;
+    have = stats ? std::min(enq, kHostStats) : 0;
+    rc = read_flow(c, have);
+    if (rc != SPM_OK || c->host_flow[FW_GO] == 0) break;
     if (spm_cancelled(c)) { rc = spm_fail(SPM_ERR_CANCELLED, "cancelled"); break; }
     chunk = std::min(chunk * 2, 256);
   }
   c->m.tol_grad = 0.0;
   if (rc != SPM_OK) return rc;
-  return spm_grad_flow_collect(c, stats, max_steps, steps_done);
+  return finish_flow(c, stats, max_steps, steps_done, have);
 }
 
 FloorWatch::FloorWatch(double switch_at, int window) : sw(switch_at), short_win(window), long_win(16 * window) {}

@@ -23,6 +23,8 @@ struct TmEntry {
   CUtensorMap map;
 };
 
+constexpr int kHostStats = 512;  // step records a context keeps room for in pinned memory
+
 struct spm_ctx {
   int N = 0;
   int prec = 0;
@@ -41,6 +43,7 @@ struct spm_ctx {
   void *buf = nullptr;      // spectral scratch, scratch_cap fields
   int scratch_cap = 0;
   double *host_scal = nullptr;  // pinned
+  double *host_stats = nullptr; // pinned, kHostStats step records
   int *host_flow = nullptr;     // pinned
   uint64_t launches = 0;
   void *extra = nullptr;        // solver state (LOBPCG / SPM work arrays)

@@ -219,7 +219,7 @@ class SpmContext:
         n = ctypes.c_int()
         check(lib().spm_grad_flow(self.h, _ptr(phi), _ptr(uhat), int(max_steps), float(tol_grad), st,
                                   ctypes.byref(n)))
-        return np.array([[s.energy, s.res, s.grad_norm, s.e1] for s in st[:n.value]]).reshape(-1, 4)
+        return np.frombuffer(st, dtype=np.float64).reshape(-1, 4)[:n.value].copy()
 
     def get_min_u_F_mixed(self, phi, uhat, max_steps: int, tol_grad: float, switch_tol: float = 0.0):
         """FP32 flow to switch_tol (0: as far as FP32 goes), then FP64 polish to tol_grad (FP64 context).
@@ -232,7 +232,7 @@ class SpmContext:
         check(f(self.h, _ptr(phi), _ptr(uhat), int(max_steps), float(tol_grad), float(switch_tol), st,
                 ctypes.byref(a), ctypes.byref(b)))
         n = a.value + b.value
-        return np.array([[s.energy, s.res, s.grad_norm, s.e1] for s in st[:n]]).reshape(-1, 4), a.value, b.value
+        return np.frombuffer(st, dtype=np.float64).reshape(-1, 4)[:n].copy(), a.value, b.value
 
     def tune(self, knob: str, value: int):
         f = lib().spm_tune
