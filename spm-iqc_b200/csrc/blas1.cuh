@@ -28,6 +28,53 @@ __global__ void __launch_bounds__(kThreads) field_reduce_kernel(const __grid_con
     F::fin(p, b, tot);
 }
 
+// get_Ene (LPsrc.cpp:8-38) of the state phi = p.in[0], u = p.st[0] (packed
+// spectrum) in one streaming pass over both: scal[SC_E2], scal[SC_E1]. A warp
+// takes a spectrum row (kx, ky); the packed column c = 0 is unpacked with the
+// first value of the row (-kx, -ky). (Through the pencil tiles the spectrum was
+// read in 32-byte runs: get_Ene at 192^3 74 us with its read-back, 60 us here.)
+template <class T> __global__ void __launch_bounds__(kThreads) energy_kernel(const __grid_constant__ KParams p, int N) {
+  __shared__ double red[32 * 2];
+  __shared__ double2 gx[129];  // symbol factors per |K|, N <= 256
+  const int M = N / 2, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i <= M; i += blockDim.x) gx[i] = __ldg(p.gtab + i);
+  __syncthreads();
+  double acc[2] = {0.0, 0.0};
+  const size_t npairs = (size_t)N * N * M;
+  const c2<T> *phi = reinterpret_cast<const c2<T> *>(p.in[0]);
+  const T mtau2 = (T)(-0.5 * p.m.Tau), mgam3 = (T)(-p.m.Gamma / 3.0);
+#pragma unroll 4
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < npairs; i += (size_t)gridDim.x * blockDim.x) {
+    const c2<T> x = __ldg(phi + i);
+    acc[0] += (double)poly_energy(x.x, mtau2, mgam3) + (double)poly_energy(x.y, mtau2, mgam3);
+  }
+  const c2<T> *u = reinterpret_cast<const c2<T> *>(p.st[0]);
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < N * N; row += warps) {
+    const int kx = row / N, ky = row % N;
+    const int ax = kx <= M ? kx : N - kx, ay = ky <= M ? ky : N - ky;
+    const double2 a = gx[ax], b = gx[ay], xy = {a.x * b.x, a.y + b.y};
+    for (int c = lane; c < M; c += 32) {
+      const c2<T> v = __ldg(u + (size_t)row * M + c);
+      const double vx = (double)v.x, vy = (double)v.y;
+      if (c) {
+        acc[1] += pair_symbol(gx[c], xy) * (vx * vx + vy * vy);  // weight 2, times 1/2
+      } else {
+        const c2<T> w = __ldg(u + ((size_t)((N - kx) % N) * N + (N - ky) % N) * M);
+        const double wx = (double)w.x, wy = (double)w.y;
+        const double ax0 = 0.5 * (vx + wx), ay0 = 0.5 * (vy - wy), axm = 0.5 * (vy + wy), aym = 0.5 * (wx - vx);
+        acc[1] += 0.5 * (pair_symbol(gx[0], xy) * (ax0 * ax0 + ay0 * ay0) +
+                         pair_symbol(gx[M], xy) * (axm * axm + aym * aym));
+      }
+    }
+  }
+  double tot[2];
+  if (grid_reduce<2, 0u>(acc, red, p.partials, p.tickets, gridDim.x, blockIdx.x, tot)) {
+    p.scal[SC_E2] = tot[0] * p.m.inv_n3;
+    p.scal[SC_E1] = tot[1];
+  }
+}
+
 // <p, q> sums (BasicOperators.cpp:132-143): in = p, aux0 = q.
 template <class T> struct ProDot {
   static constexpr int NR = 1;

@@ -8,6 +8,11 @@ namespace spm {
 
 template <class T> __device__ __forceinline__ const T *fld(const void *p) { return reinterpret_cast<const T *>(p); }
 __device__ __forceinline__ double *scal_of(const KParams &p, int b) { return p.scal + (size_t)b * kScal; }
+// A scalar that an earlier kernel has written: constant here, so that a
+// thread's points share one load (and what is computed from it).
+__device__ __forceinline__ double scal_in(const KParams &p, int b, int slot) {
+  return __ldg(p.scal + (size_t)b * kScal + slot);
+}
 
 // ===================================================================== prologues
 // Transform the field as it is; no reduction.
@@ -42,12 +47,20 @@ template <class T> struct ProGrad {
   template <class A> __device__ static c2<T> pro(const KParams &p, int b, size_t, c2<T> x, A (&acc)[1]) {
     const ModelC &m = model(p, b);
     const T tau = (T)m.Tau, gam = (T)m.Gamma;
-    const T mtau2 = (T)(-0.5 * m.Tau), mgam3 = (T)(-m.Gamma / 3.0);
-    acc[0] += (A)poly_energy(x.x, mtau2, mgam3) + (A)poly_energy(x.y, mtau2, mgam3);
-    return c2<T>{poly_force(x.x, tau, gam), poly_force(x.y, tau, gam)};
+    const c2<T> f = {poly_force(x.x, tau, gam), poly_force(x.y, tau, gam)};
+    if constexpr (sizeof(T) == 8) {
+      // from the force, -4 e(u) = u (f(u) + u (Tau + Gamma/3 u)): three operations a value instead of five
+      const T gam3 = (T)(m.Gamma / 3.0);
+      acc[0] = fma(x.x, fma(x.x, fma(gam3, x.x, tau), f.x), acc[0]);
+      acc[0] = fma(x.y, fma(x.y, fma(gam3, x.y, tau), f.y), acc[0]);
+    } else {
+      const T mtau2 = (T)(-0.5 * m.Tau), mgam3 = (T)(-m.Gamma / 3.0);
+      acc[0] += (A)poly_energy(x.x, mtau2, mgam3) + (A)poly_energy(x.y, mtau2, mgam3);
+    }
+    return f;
   }
   __device__ static void fin(const KParams &p, int b, const double (&tot)[1]) {
-    scal_of(p, b)[SC_E2] = tot[0] * model(p, b).inv_n3;
+    scal_of(p, b)[SC_E2] = (sizeof(T) == 8 ? -0.25 : 1.0) * tot[0] * model(p, b).inv_n3;
   }
 };
 
@@ -299,7 +312,7 @@ template <class T> struct OpForce {
   __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T> s, c2<T> &,
                                c2<T> &inv, double (&)[1], double) {
     const T iden = (T)sy.force();  // 1 / (1 + G)
-    const T sc = (T)scal_of(p, b)[SC_S];
+    const T sc = (T)scal_in(p, b, SC_S);
     const c2<T> fh = cscale(f, (T)S::scale(p.m));
     inv = c2<T>{(fh.x - sc * s.x) * iden, (fh.y - sc * s.y) * iden};
     if (Kx == 0 && Ky == 0 && Kz == 0) inv = c2<T>{0, 0};
@@ -318,7 +331,7 @@ template <class T, bool NORM = true> struct OpTangent {
   template <class S>
   __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T>, c2<T> &so,
                                c2<T> &inv, double (&)[1], double) {
-    const T inrm = NORM ? (T)(1.0 / sqrt(scal_of(p, b)[SC_NRM2])) : (T)1;
+    const T inrm = NORM ? (T)(1.0 / sqrt(scal_in(p, b, SC_NRM2))) : (T)1;
     const c2<T> v = cscale(cscale(f, (T)S::scale(p.m)), inrm);
     so = v;
     inv = (Kx == 0 && Ky == 0 && Kz == 0) ? c2<T>{0, 0} : cscale(v, (T)sy.G());
@@ -392,7 +405,7 @@ template <class T> struct EpiNgrad {
   template <class A> __device__ static c2<T> epi(const KParams &p, int b, size_t idx, c2<T> y, A (&acc)[1]) {
     const c2<T> ph = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
     const T tau = (T)p.m.Tau, gam = (T)p.m.Gamma;
-    const T mg = -(T)scal_of(p, b)[SC_MU];
+    const T mg = -(T)scal_in(p, b, SC_MU);
     c2<T> o;
     o.x = -((y.x - tau * ph.x - gam * (ph.x * ph.x) + ph.x * ph.x * ph.x) - mg);
     o.y = -((y.y - tau * ph.y - gam * (ph.y * ph.y) + ph.y * ph.y * ph.y) - mg);
@@ -441,7 +454,7 @@ template <class T> struct EpiHv {
   __device__ static c2<T> epi(const KParams &p, int b, size_t idx, c2<T> y, double (&)[1]) {
     const c2<T> ph = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
     const c2<T> v = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux1[b]) + idx));
-    const T tau = (T)p.m.Tau, gam = (T)p.m.Gamma, mu = (T)scal_of(p, b)[SC_MU];
+    const T tau = (T)p.m.Tau, gam = (T)p.m.Gamma, mu = (T)scal_in(p, b, SC_MU);
     return c2<T>{y.x + (-tau - (T)2 * gam * ph.x + (T)3 * ph.x * ph.x) * v.x - mu,
                  y.y + (-tau - (T)2 * gam * ph.y + (T)3 * ph.y * ph.y) * v.y - mu};
   }
@@ -458,7 +471,7 @@ template <class T> struct EpiTangent {
     if (p.sto[b]) {
       const c2<T> a = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
       const c2<T> c = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux1[b]) + idx));
-      const T d = (T)sqrt(scal_of(p, b)[SC_NRM2]);
+      const T d = (T)sqrt(scal_in(p, b, SC_NRM2));
       *reinterpret_cast<c2<T> *>(reinterpret_cast<T *>(p.sto[b]) + idx) = c2<T>{(c.x - a.x) / d, (c.y - a.y) / d};
     }
     return y;
@@ -484,7 +497,7 @@ template <class T> struct EpiPrecond {
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
   __device__ static c2<T> epi(const KParams &p, int b, size_t, c2<T> y, double (&)[1]) {
-    const T mu = (T)scal_of(p, b)[SC_MU];
+    const T mu = (T)scal_in(p, b, SC_MU);
     return c2<T>{y.x - mu, y.y - mu};
   }
   __device__ static void fin(const KParams &, int, const double (&)[1]) {}

@@ -114,12 +114,14 @@ template <int N, class T> struct Impl {
 
   // E2 -> scal[SC_E2], E1 -> scal[SC_E1]
   static int energy(spm_ctx *c, const void *phi, const void *uhat) {
+    if (((uintptr_t)uhat & 15u) != 0) return spm_fail(SPM_ERR_ARG, "spectrum buffers must be 16-byte aligned");
     KParams p = spm_params(c);
     p.in[0] = phi;
-    SPM_TRY((reduce<N, T, ProGrad<T>>(c, p, 1)));
-    KParams q = spm_params(c);
-    q.st[0] = uhat;
-    return pencil<N, T, OpE1<T>>(c, q, 1);
+    p.st[0] = uhat;
+    c->launches++;
+    energy_kernel<T><<<N >= 128 ? kReduceBlocks : kReduceBlocks / 4, kThreads, 0, c->stream>>>(p, N);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : spm_fail_cuda(e, "energy");
   }
 
   // One semi-implicit step of three passes, gated by the flow words. With ev
@@ -329,7 +331,7 @@ template <int N, class T> struct Impl {
   // Tangent preparation (get_Tv, SPM.cpp:15-32, plus what the force steps
   // need): with phi0 set, d = phi1 - phi0 is normalised and v = d/||d|| is
   // written to v_out; with phi0 null, phi1 is the tangent as given. Always
-  // writes vhat = FFT(v)/N^3 (packed) and Gv = IFFT(G vhat, k = 0 removed).
+  // writes vhat = FFT(v)/N^3 (in tile order, state_index) and Gv = IFFT(G vhat, k = 0 removed).
   static int tangent(spm_ctx *c, const void *phi0, const void *phi1, void *v_out, void *vhat, void *gv) {
     SPM_NEED_SCRATCH(c, 1);
     KParams p = spm_params(c);
@@ -340,6 +342,7 @@ template <int N, class T> struct Impl {
     KParams q = spm_params(c);
     q.in[0] = spm_buf(c, 0);
     q.sto[0] = vhat;
+    q.sto_tiled = 1;
     q.out[0] = spm_buf(c, 0);
     if (phi0) SPM_TRY((pencil<N, T, OpTangent<T, true>>(c, q, 1)));
     else SPM_TRY((pencil<N, T, OpTangent<T, false>>(c, q, 1)));
@@ -359,6 +362,7 @@ template <int N, class T> struct Impl {
     SPM_NEED_SCRATCH(c, n);
     KParams p = spm_params(c), q = spm_params(c), r = spm_params(c);
     p.m.factor = factor;
+    q.st_tiled = 1;
     for (int b = 0; b < n; b++) {
       p.in[b] = x[b];
       p.aux0[b] = v;

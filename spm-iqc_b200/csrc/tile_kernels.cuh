@@ -762,6 +762,7 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
     const bool packed = !Op::LIN && col == 0;
     constexpr int SG = M1 <= 8 ? M1 : M1 / 2;  // state loads in flight per thread
     auto points = [&](auto &a) {
+      if (!Op::LIN) __builtin_assume(col > 0);
 #pragma unroll
       for (int h = 0; h < M1; h += SG) {
         T2 s[SG];
