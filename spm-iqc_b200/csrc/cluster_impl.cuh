@@ -21,7 +21,7 @@ namespace clu {
 // while the previous kernel of the stream finishes, and wait for it in
 // grid_dep_sync.
 template <class Tag, int N, class K, int RW = kRows>
-static int launch_cluster(spm_ctx *c, K kern, size_t smem, const KParamsC &p, int nb, const char *what,
+static int launch_cluster(spm_ctx *c, K kern, size_t smem, KParamsC &p, int nb, const char *what,
                           bool xg = false, int regions = 2) {
   constexpr int CLr = N / RW;
   cudaError_t e = prepare<Tag>(kern, smem, c->device);
@@ -61,7 +61,10 @@ static int launch_cluster(spm_ctx *c, K kern, size_t smem, const KParamsC &p, in
     ncl[dev].store(nc, std::memory_order_relaxed);
   }
   cfg.gridDim = dim3(CLr * nc, nb, 1);
-  cfg.numAttrs = pdl_on(c) ? 2 : 1;  // the kernels begin with grid_dep_sync
+  // a grid with a plane per cluster, all of them resident, lets the next launch
+  // in while it runs (grid_dep_trigger)
+  p.trigger = nc == N && nb == 1;
+  cfg.numAttrs = pdl_on(c) || p.trigger ? 2 : 1;  // the kernels begin with grid_dep_sync
   // a kernel exchanging through global areas needs one per CTA (nb == 1)
   if (xg && (!p.xg || nb != 1 || CLr * nc > p.xg_cap * (kRows / RW) || p.xg_regions < regions))
     return spm_fail(SPM_ERR_STATE, "plane exchange areas missing or too small");
@@ -89,7 +92,7 @@ template <class T> static inline bool cps4(const spm_ctx *c) { return sizeof(T) 
 // The plane kernels come in four variants (c->plane_cps): 1 = staged, one CTA
 // per SM; 2 = direct loads, two CTAs per SM; 3 = direct, three CTAs per SM;
 // 4 = direct, four CTAs per SM for FP32 gradient chains (3 elsewhere).
-template <int N, class T, class Pro> static int plane_fwd(spm_ctx *c, const KParamsC &p, int nb) {
+template <int N, class T, class Pro> static int plane_fwd(spm_ctx *c, KParamsC &p, int nb) {
   if constexpr (XgOk<Pro>::value) {
     if (xg_bits(c, nb) & kXgFwd) {
       if (rw16(c, nb)) {
@@ -125,7 +128,7 @@ template <int N, class T, class Pro> static int plane_fwd(spm_ctx *c, const KPar
   struct Tag1 {};
   return launch_cluster<Tag1, N>(c, plane_fwd_kernel<N, T, Pro, 1>, plane_smem<N, T, 1>(), p, nb, "plane_fwd");
 }
-template <int N, class T, class Epi> static int plane_inv(spm_ctx *c, const KParamsC &p0, int nb) {
+template <int N, class T, class Epi> static int plane_inv(spm_ctx *c, KParamsC &p0, int nb) {
   if constexpr (XgOk<Epi>::value) {
     if (xg_bits(c, nb) & kXgInv) {
       if (rw16(c, nb)) {
@@ -166,7 +169,7 @@ template <int N, class T, class Epi> static int plane_inv(spm_ctx *c, const KPar
 // The fused inverse -> forward plane pass (direct loads; two CTAs per SM, or
 // three with plane_cps = 3), with the exchange routes XG.
 template <int N, class T, class Epi, class Pro, int XG>
-static int plane_inv_fwd_xg(spm_ctx *c, const KParamsC &p, int nb) {
+static int plane_inv_fwd_xg(spm_ctx *c, KParamsC &p, int nb) {
   if constexpr (sizeof(T) == 4 && XG != 0) {
     if (cps4<T>(c)) {
       struct Tag4 {};
@@ -183,7 +186,7 @@ static int plane_inv_fwd_xg(spm_ctx *c, const KParamsC &p, int nb) {
   return launch_cluster<Tag2, N>(c, plane_inv_fwd_kernel<N, T, Epi, Pro, 2, XG>, plane_smem<N, T, 2>(), p, nb,
                                  "plane_inv_fwd", XG != 0);
 }
-template <int N, class T, class Epi, class Pro> static int plane_inv_fwd(spm_ctx *c, const KParamsC &p, int nb) {
+template <int N, class T, class Epi, class Pro> static int plane_inv_fwd(spm_ctx *c, KParamsC &p, int nb) {
   if constexpr (XgOk<Pro>::value && XgOk<Epi>::value) {
     if (rw16(c, nb)) {
       constexpr int XG = kXgFwd | kXgInv;
@@ -208,7 +211,7 @@ template <int N, class T, class Epi, class Pro> static int plane_inv_fwd(spm_ctx
 }
 // Persistent pencil launch: resident CTAs (queried once), at most one per tile;
 // tiles of 8 columns, or 4 (knob "pencil_tc"); programmatic dependent with pdl_on.
-template <int N, class T, class Op, int TC> static int pencil_tc(spm_ctx *c, const KParamsC &p0, int nb) {
+template <int N, class T, class Op, int TC> static int pencil_tc(spm_ctx *c, KParamsC &p0, int nb) {
   using PG = PencilGeo<N, TC>;
   KParamsC p = p0;
   const int kind = TC == 8 ? TM_PENCIL : TM_PENCIL4;
@@ -243,12 +246,13 @@ template <int N, class T, class Op, int TC> static int pencil_tc(spm_ctx *c, con
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pdl_on(c) ? 1 : 0;  // the kernel begins with grid_dep_sync
+  p.trigger = nbk == PG::PTILES && nb == 1;
+  cfg.numAttrs = pdl_on(c) || p.trigger ? 1 : 0;  // the kernel begins with grid_dep_sync
   c->launches++;
   e = cudaLaunchKernelEx(&cfg, kern, p);
   return e == cudaSuccess ? 0 : spm_fail_cuda(e, "pencil launch");
 }
-template <int N, class T, class Op> static int pencil(spm_ctx *c, const KParamsC &p, int nb) {
+template <int N, class T, class Op> static int pencil(spm_ctx *c, KParamsC &p, int nb) {
   if (c->pencil_tc == 4) return pencil_tc<N, T, Op, 4>(c, p, nb);
   return pencil_tc<N, T, Op, 8>(c, p, nb);
 }

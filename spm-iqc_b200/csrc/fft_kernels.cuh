@@ -466,6 +466,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_fwd_kernel(const __grid_con
   double *red = reinterpret_cast<double *>(bar + 2);
   __shared__ int s_err;
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -576,6 +577,7 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
   double2 *stab = reinterpret_cast<double2 *>(red + 32 * kRedMax);  // symbol buffers (one or two tiles)
   __shared__ int s_err;
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -829,6 +831,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_kernel(const __grid_con
   double *red = reinterpret_cast<double *>(bar + 2);
   __shared__ int s_err;
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -927,6 +930,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_kernel(const __grid
   uint64_t *bar = reinterpret_cast<uint64_t *>(buf + P::UNITS);
   double *red = reinterpret_cast<double *>(bar + 2);
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
   // uniform over the grid: set by the pencil pass of this step, before launch
   const bool stop = flow_pending(p, blockIdx.y);
@@ -1054,6 +1058,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_fwd_pipe_kernel(const _
   uint64_t *bar = reinterpret_cast<uint64_t *>(buf + P::UNITS);
   double *red = reinterpret_cast<double *>(bar + 2);
   grid_dep_sync();
+  if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, blockIdx.y)) return;
   const bool stop = flow_pending(p, blockIdx.y);
 

@@ -17,10 +17,10 @@ namespace spm {
 // load), so the reductions' partial sums, and hence the results, do not
 // either. With pdl_on the launch is a programmatic dependent one: it may be set
 // up while the previous kernel of the stream finishes, and waits for it in
-// grid_dep_sync. Grids of at most half of the resident blocks (all but a few
-// of the batched ones up to 96^3) are launched that way in any case, and let the next
-// launch in as soon as they run: its blocks are then placed, with their
-// twiddles loaded, when this one completes.
+// grid_dep_sync. Grids that are resident at once with a tile per block (plane
+// passes up to 128^3, pencil passes up to 64^3) are launched that way in any
+// case, and let the next launch in as soon as they run: its blocks are then
+// placed, with their twiddles loaded, when this one completes.
 template <class Tag, class K, class P>
 static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles, P &p, int nb, const char *what) {
   cudaError_t e = prepare<Tag>(kern, smem, c->device);
@@ -38,7 +38,7 @@ static int launch_tiles(spm_ctx *c, K kern, int threads, size_t smem, int tiles,
     resident[dev].store(most, std::memory_order_relaxed);
   }
   const int nbk = std::min({most, tiles, kPartStride});
-  p.trigger = 2 * nbk * nb <= most;
+  p.trigger = nbk == tiles && nbk * nb <= most;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nb, nbk, 1);
   cfg.blockDim = dim3(threads, 1, 1);
