@@ -274,11 +274,12 @@ __global__ void __launch_bounds__((kStageWarps + 1) * 32, 1) gram_staged_kernel(
       }
   }
   __syncthreads();
-  double *part = p.partials + (size_t)blockIdx.x * kBlkMax * kBlkMax;
-  for (int e = tid; e < RA * RB; e += NW * 32) {
+  constexpr int NE = RA * RB;
+  double *part = p.partials + (size_t)blockIdx.x * NE;
+  for (int e = tid; e < NE; e += NW * 32) {
     double s = 0.0;
-    for (int w = 0; w < kStageWarps; w++) s += tile[w * RA * RB + e];
-    part[(e / RB) * kBlkMax + e % RB] = s;
+    for (int w = 0; w < kStageWarps; w++) s += tile[w * NE + e];
+    part[e] = s;
   }
   if (tid == 0 && s_err) atomicExch(p.err, 1);
   __threadfence();
@@ -287,16 +288,26 @@ __global__ void __launch_bounds__((kStageWarps + 1) * 32, 1) gram_staged_kernel(
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // grid total of every entry in a fixed order (as gram_kernel)
-  for (int e = warp; e < p.ma * p.mb; e += NW) {
-    const int r = e / p.mb, c = e % p.mb;
-    double s = 0.0;
-#pragma unroll 4
-    for (unsigned bk = lane; bk < gridDim.x; bk += 32)
-      s += __ldcg(p.partials + (size_t)bk * kBlkMax * kBlkMax + r * kBlkMax + c);
+  // Grid total of every entry in a fixed order by the last CTA (the order of
+  // gram_kernel: 32 sums over every 32nd CTA, then their binary tree), one
+  // thread per entry: consecutive threads read consecutive entries, with 32 loads
+  // in flight each. (A warp per entry and a lane per CTA read a sector per value:
+  // 64 us for 24 x 24 entries; the 24-field Gram pair at 128^3 198 -> 157 us.)
+  for (int e = tid; e < NE; e += NW * 32) {
+    double s[32];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) p.out[e] = s * p.inv_n;
+    for (int l = 0; l < 32; l++) s[l] = 0.0;
+#pragma unroll 1
+    for (unsigned bk = 0; bk < gridDim.x; bk += 32)
+#pragma unroll
+      for (int l = 0; l < 32; l++)
+        if (bk + l < gridDim.x) s[l] += __ldcg(p.partials + (size_t)(bk + l) * NE + e);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+      for (int l = 0; l < off; l++) s[l] += s[l + off];
+    const int r = e / RB, c = e % RB;
+    if (r < p.ma && c < p.mb) p.out[r * p.mb + c] = s[0] * p.inv_n;
   }
   if (tid == 0) {
     p.out[p.ma * p.mb] = (double)*((volatile int *)p.err);
@@ -503,18 +514,22 @@ __global__ void __launch_bounds__((kCombWarps + 1) * 32, 1) combine_staged_kerne
     }
   }
   if (!p.norms) return;
-  // the outputs' squared norms: per CTA in a fixed thread order, then over
-  // the CTAs in a fixed order by the last CTA
+  // the outputs' squared norms, in a fixed order: over a warp's lanes, the
+  // warps, then the CTAs by the last CTA (a warp per output; one thread per
+  // output over all threads, then over all CTAs, cost 30 us)
   __syncthreads();
-  double *red = reinterpret_cast<double *>(st);  // [threads][NO], over the idle ring
-  const int nthr = (kCombWarps + 1) * 32;
+  double *red = reinterpret_cast<double *>(st);  // [warps][NO], over the idle ring
 #pragma unroll
-  for (int q = 0; q < NO; q++) red[(size_t)tid * NO + q] = nsq[q];
+  for (int q = 0; q < NO; q++) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) nsq[q] += __shfl_xor_sync(0xffffffffu, nsq[q], off);
+    if (lane == 0) red[warp * NO + q] = nsq[q];
+  }
   __syncthreads();
   __shared__ int s_last;
   if (tid < NO) {
     double t = 0.0;
-    for (int u = 0; u < nthr; u++) t += red[(size_t)u * NO + tid];
+    for (int w = 0; w < kCombWarps + 1; w++) t += red[w * NO + tid];
     p.partials[(size_t)blockIdx.x * kBlkMax + tid] = t;
   }
   __threadfence();
@@ -523,10 +538,13 @@ __global__ void __launch_bounds__((kCombWarps + 1) * 32, 1) combine_staged_kerne
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  if (tid < NO && tid < p.nout) {
+  if (warp < NO && warp < p.nout) {
     double t = 0.0;
-    for (unsigned bk = 0; bk < gridDim.x; bk++) t += __ldcg(p.partials + (size_t)bk * kBlkMax + tid);
-    p.norms[tid] = t * p.inv_n;
+#pragma unroll 8
+    for (unsigned bk = lane; bk < gridDim.x; bk += 32) t += __ldcg(p.partials + (size_t)bk * kBlkMax + warp);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+    if (lane == 0) p.norms[warp] = t * p.inv_n;
   }
   if (tid == 0) {
     p.norms[p.nout] = (double)*((volatile int *)p.err);
