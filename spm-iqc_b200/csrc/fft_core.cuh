@@ -285,13 +285,15 @@ __device__ __forceinline__ void block_reduce(double (&a)[NR], double *scratch, i
   }
 }
 
-// Grid reduction: every group writes its total to partials[bidx]; the group
-// that finishes last sums all nblk partials in fixed index order (so the result
-// does not depend on scheduling) and returns true in its thread 0 with tot filled.
+// Grid reduction in two halves: every group writes its total to partials[bidx]
+// and takes a ticket (group_arrive); the group with the last one sums all nblk
+// partials in fixed index order (so the result does not depend on scheduling) and
+// returns true in its thread 0 with tot filled (group_finish). Between the
+// halves a kernel runs what does not change acc: the ticket's round trip to L2
+// is then hidden.
 template <int NR, unsigned MAXM, int G>
-__device__ __forceinline__ bool group_reduce(double (&acc)[NR], double *scratch, double *partials, unsigned *ticket,
-                                             int nblk, int bidx, int g, int tid, int nth, double (&tot)[NR]) {
-  __shared__ int s_last[G];
+__device__ __forceinline__ void group_arrive(double (&acc)[NR], double *scratch, double *partials, unsigned *ticket,
+                                             int nblk, int bidx, int g, int tid, int nth, int *s_last) {
   block_reduce<NR, MAXM, G>(acc, scratch, g, tid, nth);
   if (tid == 0) {
 #pragma unroll
@@ -300,6 +302,10 @@ __device__ __forceinline__ bool group_reduce(double (&acc)[NR], double *scratch,
     unsigned prev = atomicAdd(ticket, 1u);
     s_last[g] = (prev == (unsigned)nblk - 1u);
   }
+}
+template <int NR, unsigned MAXM, int G>
+__device__ __forceinline__ bool group_finish(double *scratch, double *partials, unsigned *ticket, int nblk, int g,
+                                             int tid, int nth, const int *s_last, double (&tot)[NR]) {
   group_sync<G>(g, nth);
   if (!s_last[g]) return false;
   __threadfence();
@@ -325,7 +331,9 @@ __device__ __forceinline__ bool group_reduce(double (&acc)[NR], double *scratch,
 template <int NR, unsigned MAXM>
 __device__ __forceinline__ bool grid_reduce(double (&acc)[NR], double *scratch, double *partials,
                                             unsigned *ticket, int nblk, int bidx, double (&tot)[NR]) {
-  return group_reduce<NR, MAXM, 1>(acc, scratch, partials, ticket, nblk, bidx, 0, threadIdx.x, blockDim.x, tot);
+  __shared__ int s_last[1];
+  group_arrive<NR, MAXM, 1>(acc, scratch, partials, ticket, nblk, bidx, 0, threadIdx.x, blockDim.x, s_last);
+  return group_finish<NR, MAXM, 1>(scratch, partials, ticket, nblk, 0, threadIdx.x, blockDim.x, s_last, tot);
 }
 
 // ------------------------------------------------------------------ async copies
@@ -595,6 +603,15 @@ __device__ __forceinline__ double *stats_of(const KParams &p, int b) { return p.
 __device__ __forceinline__ bool flow_stopped(const KParams &p, int b) {
   const int *f = flow_of(p, b);
   return f != nullptr && *((volatile const int *)f + FW_GO) == 0;
+}
+// Both words in one load: returns flow_stopped, sets pending.
+__device__ __forceinline__ bool flow_state(const KParams &p, int b, bool &pending) {
+  static_assert(FW_GO == 0 && FW_PENDING == 1, "one 8-byte load");
+  const int *f = flow_of(p, b);
+  if (f == nullptr) return false;
+  const int2 w = __ldcg(reinterpret_cast<const int2 *>(f));
+  pending = w.y != 0;
+  return w.x == 0;
 }
 // The step's stop is armed (FW_PENDING, set by its pencil pass before launch).
 __device__ __forceinline__ bool flow_pending(const KParams &p, int b) {

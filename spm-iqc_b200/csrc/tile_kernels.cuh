@@ -416,13 +416,19 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
       report_error(p, *st.err);
     }
   }
-  // Grid reduction over the threads of every group (grid_reduce); fin(tot) runs
-  // in one thread.
-  template <int NR, unsigned MAXM, class F>
-  __device__ void reduce(const KParams &p, int b, double (&acc)[NR], F fin) {
+  // The tile is the last one of this thread's group.
+  __device__ bool last(int x, int j2) const { return x * P::YB + j2 + G * block_count() >= PG::TILES; }
+  // Grid reduction over the groups: arrive once acc is complete, finish at the end
+  // of the kernel; fin(tot) runs in one thread.
+  template <int NR, unsigned MAXM> __device__ void arrive(const KParams &p, int b, double (&acc)[NR], int *s_last) {
+    group_arrive<NR, MAXM, G>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax, p.tickets + b,
+                              G * block_count(), block_id() + g * block_count(), g, tid, G > 1 ? N : blockDim.x,
+                              s_last);
+  }
+  template <int NR, unsigned MAXM, class F> __device__ void finish(const KParams &p, int b, const int *s_last, F fin) {
     double tot[NR];
-    if (group_reduce<NR, MAXM, G>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax, p.tickets + b,
-                                  G * block_count(), block_id() + g * block_count(), g, tid, G > 1 ? N : blockDim.x, tot))
+    if (group_finish<NR, MAXM, G>(red, p.partials + (size_t)b * kPartStride * kRedMax, p.tickets + b,
+                                  G * block_count(), g, tid, G > 1 ? N : blockDim.x, s_last, tot))
       fin(tot);
   }
 };
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(N, PlaneGeo<N, T>::CPS)
   using P = Plane<N, T>;
   constexpr int N1 = P::N1, YB = P::YB;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_err;
+  __shared__ int s_err, s_last[1];
   PlaneLoop<N, T, false, 1> loop(smem_raw, &s_err);
   T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
@@ -491,6 +497,8 @@ __global__ void __launch_bounds__(N, PlaneGeo<N, T>::CPS)
           acc);
       P::row_store_fwd(buf, r, jz, v);
     });
+    if constexpr (Pro::NR > 0)
+      if (loop.last(x, j2)) loop.template arrive<Pro::NR, Pro::MAXM>(p, b, acc, s_last);
     loop.sync();
     P::class_fwd(buf, tw, tid);
     loop.sync();
@@ -498,7 +506,7 @@ __global__ void __launch_bounds__(N, PlaneGeo<N, T>::CPS)
     loop.sync();
   });
   if constexpr (Pro::NR > 0)
-    loop.template reduce<Pro::NR, Pro::MAXM>(p, b, acc, [&](double (&tot)[Pro::NR]) { Pro::fin(p, b, tot); });
+    loop.template finish<Pro::NR, Pro::MAXM>(p, b, s_last, [&](double (&tot)[Pro::NR]) { Pro::fin(p, b, tot); });
 }
 
 // --------------------------------------------------------------- plane_inv
@@ -515,7 +523,7 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
   constexpr int G = inv_groups<N, T>();
   constexpr int N1 = P::N1, YB = P::YB;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_err;
+  __shared__ int s_err, s_last[G];
   PlaneLoop<N, T, true, G> loop(smem_raw, &s_err);
   T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
@@ -544,8 +552,10 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
     });
     loop.sync();
   });
-  if constexpr (Epi::NR > 0)
-    loop.template reduce<Epi::NR, Epi::MAXM>(p, b, acc, [&](double (&tot)[Epi::NR]) { Epi::fin(p, b, tot); });
+  if constexpr (Epi::NR > 0) {
+    loop.template arrive<Epi::NR, Epi::MAXM>(p, b, acc, s_last);
+    loop.template finish<Epi::NR, Epi::MAXM>(p, b, s_last, [&](double (&tot)[Epi::NR]) { Epi::fin(p, b, tot); });
+  }
 }
 
 // --------------------------------------------------------------- plane_inv_fwd
@@ -564,16 +574,17 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
   constexpr int N1 = P::N1, YB = P::YB;
   constexpr int NE = Epi::NR, NP = Pro::NR, NA = (NE + NP > 0) ? NE + NP : 1;
   static_assert(NA <= kRedMax, "reduction count");
+  constexpr unsigned MAXM = Epi::MAXM | (Pro::MAXM << NE);
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_err;
+  __shared__ int s_err, s_last[G];
   PlaneLoop<N, T, true, G> loop(smem_raw, &s_err);
   T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
-  if (flow_stopped(p, field_id())) return;
   // uniform over the grid: set by the pencil pass of this step, before launch
-  const bool stop = flow_pending(p, field_id());
+  bool stop = false;
+  if (flow_state(p, field_id(), stop)) return;
   const int tid = loop.tid, b = field_id();
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
   T *phi = reinterpret_cast<T *>(p.sto[b]);
@@ -604,6 +615,15 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
           acc_p);
       P::row_store_fwd(buf, r, jz, v);
     });
+    if (loop.last(x, j2)) {
+      double all[NA];
+#pragma unroll
+      for (int r = 0; r < NE; r++) all[r] = acc_e[r];
+#pragma unroll
+      for (int r = 0; r < NP; r++) all[NE + r] = acc_p[r];
+      if constexpr (NE + NP == 0) all[0] = 0.0;
+      loop.template arrive<NA, MAXM>(p, b, all, s_last);
+    }
     loop.sync();
     if (!stop) {
       P::class_fwd(buf, tw, tid);
@@ -622,13 +642,7 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
         u[(size_t)row * M + c] = ut[state_index<N, T>(ky % 32, ky / 32, kx, c, 1)];
     }
   }
-  double all[NA];
-#pragma unroll
-  for (int r = 0; r < NE; r++) all[r] = acc_e[r];
-#pragma unroll
-  for (int r = 0; r < NP; r++) all[NE + r] = acc_p[r];
-  if constexpr (NE + NP == 0) all[0] = 0.0;
-  loop.template reduce<NA, (Epi::MAXM | (Pro::MAXM << NE))>(p, b, all, [&](double (&tot)[NA]) {
+  loop.template finish<NA, MAXM>(p, b, s_last, [&](double (&tot)[NA]) {
     double te[NE > 0 ? NE : 1], tp[NP > 0 ? NP : 1];
 #pragma unroll
     for (int r = 0; r < NE; r++) te[r] = tot[r];
@@ -672,6 +686,7 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
   using G = Geo<N>;
   using PG = PencilGeo<N, T>;
   using T2 = c2<T>;
+  __shared__ int s_last[1];
   constexpr int R = kRun;
   constexpr int M = G::M, M1 = G::M1, YB = G::YB, C = PG::C, TH = PG::TH, KS = PG::KS, JS = PG::JS, NCG = PG::NCG;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -844,6 +859,10 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
         F[k] = kp[k];
       }
     }
+    if constexpr (Op::NR > 0)
+      if (v + block_count() >= PG::TILES)  // the block's last tile
+        group_arrive<Op::NR, Op::MAXM, 1>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax, p.tickets + b,
+                                          block_count(), block_id(), 0, tid, TH, s_last);
     if constexpr (Op::INV) {
       Dft<+1, M1, T2>::run(F);
       sfor<0, M1>([&](auto J) { ex[kb * JS + ka * KS + SPM_CI(J) * C + cc] = F[SPM_CI(J)]; });
@@ -876,8 +895,8 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
   }
   if constexpr (Op::NR > 0) {
     double tot[Op::NR];
-    if (grid_reduce<Op::NR, Op::MAXM>(acc, red, p.partials + (size_t)b * kPartStride * kRedMax,
-                                      p.tickets + b, block_count(), block_id(), tot))
+    if (group_finish<Op::NR, Op::MAXM, 1>(red, p.partials + (size_t)b * kPartStride * kRedMax, p.tickets + b,
+                                          block_count(), 0, tid, TH, s_last, tot))
       Op::fin(p, b, tot);
   }
 }
