@@ -457,6 +457,17 @@ __device__ __forceinline__ float2 ld_state(const float2 *p) {
   asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
   return v;
 }
+// The same with an L2 policy.
+__device__ __forceinline__ double2 ld_state(const double2 *p, uint64_t pol) {
+  double2 v;
+  asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
+  return v;
+}
+__device__ __forceinline__ float2 ld_state(const float2 *p, uint64_t pol) {
+  float2 v;
+  asm volatile("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+  return v;
+}
 __device__ __forceinline__ void st_stream(double2 *p, double2 v, uint64_t pol) { st_keep(p, v, pol); }
 __device__ __forceinline__ void st_stream(float2 *p, float2 v, uint64_t pol) { st_keep(p, v, pol); }
 

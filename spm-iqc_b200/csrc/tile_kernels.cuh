@@ -74,6 +74,15 @@ template <int N, class T> __device__ __forceinline__ size_t state_kx_stride(int 
 // the L1 too small for the state's loads).
 template <int N, class T> constexpr int inv_groups() { return sizeof(T) == 8 && N == 256 ? 2 : 1; }
 
+// The states of a pencil pass carry an L2 evict-first policy where the scratch
+// fits in the 126 MB L2 but not beside a state of its size (FP64: 192^3, 2 x 57
+// MB): the scratch then stays. Measured (gradient step, without and with): 192^3
+// 108 and 104 us; 256^3, whose scratch does not fit by itself, 225 and 239 us.
+template <int N, class T> constexpr bool stream_state() {
+  constexpr size_t S = sizeof(T) * (size_t)N * N * N;
+  return S < ((size_t)100 << 20) && 2 * S > ((size_t)100 << 20);
+}
+
 // Plane pass: N threads per tile of 32 rows x M complex values (16 per
 // thread), rows padded by one value. 512 threads per SM in FP64 (up to 128
 // registers each), 1024 in FP32. G: groups per block (inv_groups).
@@ -776,20 +785,28 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
     auto sym = [&](int Kx, double2 yz) { return SymFn{Op::SYM ? pair_symbol(gx[Kx < 0 ? -Kx : Kx], yz) : 0.0}; };
     const bool packed = !Op::LIN && col == 0;
     constexpr int SG = M1 <= 8 ? M1 : M1 / 2;  // state loads in flight per thread
+    constexpr bool STREAM = stream_state<N, T>();
+    const uint64_t spol = STREAM ? l2_stream_policy() : 0;
     auto points = [&](auto &a) {
       if (!Op::LIN) __builtin_assume(col > 0);
 #pragma unroll
       for (int h = 0; h < M1; h += SG) {
         T2 s[SG];
 #pragma unroll
-        for (int i = 0; i < SG; i++) s[i] = Op::SI ? ld_state(st + s0 + (h + i) * ss) : T2{0, 0};
+        for (int i = 0; i < SG; i++) {
+          const T2 *q = st + s0 + (h + i) * ss;
+          s[i] = !Op::SI ? T2{0, 0} : STREAM ? ld_state(q, spol) : ld_state(q);
+        }
 #pragma unroll
         for (int i = 0; i < SG; i++) {
           const int k = h + i, Kx = wave(ka + 16 * k, N);
           const T2 f = Op::FI ? F[k] : T2{0, 0};
           T2 o_st = {0, 0}, o_inv = {0, 0};
           Op::point(p, b, Kx, Ky, col, sym(Kx, gyz), f, s[i], o_st, o_inv, a, 2.0);
-          if constexpr (Op::SO) sto[t0 + k * ts] = o_st;
+          if constexpr (Op::SO) {
+            if constexpr (STREAM) st_stream(sto + t0 + k * ts, o_st, spol);
+            else sto[t0 + k * ts] = o_st;
+          }
           F[k] = o_inv;
         }
       }

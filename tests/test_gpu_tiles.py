@@ -67,3 +67,41 @@ def test_chain_stopping_inside_returns_its_state(cuda, N):
     back = ctx.my_fft(p)
     assert rel(back.cpu().numpy(), u.cpu().numpy()) < 1e-11
     ctx.close()
+
+
+@pytest.mark.parametrize("N", SIZES)
+def test_energy_matches_oracle(cuda, N):
+    """get_Ene streams the field and the packed spectrum (its c = 0 column
+    unpacked with partner rows). Bar: a few roundings a term and a tree of sums,
+    2^-53 * 40 log2(N^3) < 1.1e-13 of the terms' absolute sum, which is at most ten times
+    the energy for this field: 1e-12."""
+    import spmiqc
+    m = npo.Model(N, L=19.7, Tau=-0.05)
+    c = spmiqc.SpmContext(N, L=19.7, Tau=-0.05)
+    phi = npo.uniform_field(N, 5, amp=0.4)
+    pd = cuda.from_numpy(phi).cuda()
+    e, ref = c.get_Ene(pd, c.my_fft(pd)), m.energy(phi, m.my_fft(phi))
+    assert abs(e - ref) < 1e-12 * abs(ref)
+    c.close()
+
+
+def test_many_groups_run_through_a_graph(cuda):
+    """Nine instances with launches of their own (batch_group 0) go through the
+    captured graph, the same nine in one group are launched directly: the same
+    steps and fields."""
+    import spmiqc
+    out = []
+    for group in (0, 1):
+        cs = [spmiqc.SpmContext(32, L=18.0 + i, Tau=-0.002 * i) for i in range(9)]
+        for c in cs:
+            c.tune("batch_group", group)
+        ps = [cuda.from_numpy(npo.uniform_field(32, 100 + i)).cuda() for i in range(9)]
+        us = [c.my_fft(p) for c, p in zip(cs, ps)]
+        cuda.cuda.synchronize()
+        out.append((spmiqc.batch_grad_flow(cs, ps, us, 70, 1e-12, steps_per_launch=16), ps, us))
+        for c in cs:
+            c.close()
+    (d0, p0, u0), (d1, p1, u1) = out
+    assert d0 == d1 == [70] * 9
+    for a, b in zip(p0 + u0, p1 + u1):
+        assert cuda.equal(a, b)
