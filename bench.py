@@ -688,7 +688,7 @@ def main():
     ap.add_argument("--no-configs", action="store_true", help="skip the config2 / config3 legs")
     ap.add_argument("--schedule", default=None,
                     help="plane_cps,fuse_planes,plane_xg for the FP64 context instead of the autotuner's choice "
-                         "(fixed kernel variants for ncu captures)")
+                         "(fuse_planes 0 or 1; the FP64 kernels have no other variants)")
     ap.add_argument("--tune", action="append", default=[], metavar="KNOB=V",
                     help="set a tuning knob (spm_tune) of the flow contexts before the autotuner runs, e.g. pdl=0")
     ap.add_argument("--serve", action="store_true", help="run the serving workload instead (one JSON line)")

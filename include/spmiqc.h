@@ -184,10 +184,10 @@ int spm_grad_flow_mixed(spm_ctx *ctx, void *phi, void *uhat, int max_steps, doub
                         spm_step_stats *stats, int *steps_fp32, int *steps_fp64);
 
 /* Batched get_min_u_F over n independent instances (no counterpart in the
- * reference; each context may have its own N, L, Tau, Gamma, dt): one
- * captured CUDA graph advances every instance by steps_per_launch gated steps
- * on parallel stream branches and is relaunched until all instances reached
- * ||grad F|| <= tol_grad (or max_steps). With switch_tol > tol_grad the
+ * reference; each context may have its own N, L, Tau, Gamma, dt):
+ * rounds of steps_per_launch gated steps of every instance, on parallel
+ * streams (or, for many groups of instances, one captured CUDA graph), until
+ * all instances reached ||grad F|| <= tol_grad (or max_steps). With switch_tol > tol_grad the
  * instances (FP64 contexts) first run with FP32 transforms to switch_tol (or
  * until 512 FP32 steps bring no new minimum of ||grad F||), then in FP64 with
  * the steps each has left. steps_done (host, n entries, may be NULL) receives

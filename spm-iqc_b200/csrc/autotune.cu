@@ -1,6 +1,7 @@
 // Autotuner for the transform schedule of a context (no counterpart in the
 // reference; FFTW's plan search plays this role there, My_FFT.cpp:49-97).
-// Candidates: the plane-pass variant (staged with one CTA per SM, direct loads
+// FP64 contexts (tile passes): programmatic dependent launches or not (knob
+// "pdl"). FP32 contexts (cluster passes): the plane-pass variant (staged with one CTA per SM, direct loads
 // with two CTAs per SM, or three CTAs per SM with fewer registers per thread),
 // whether gradient chains use the fused inverse -> forward plane pass, and
 // whether their plane kernels exchange through distributed shared memory or
