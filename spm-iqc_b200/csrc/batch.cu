@@ -123,10 +123,14 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   for (int i = 0; i < n; i++) ctx[i]->stream = s0;
-  if (!direct) {
-    // one step of every group outside the capture sets up kernel attributes
-    // and tensor maps; it counts as the first step of the flow
+  // One step of every group ahead of the rounds: outside the capture it sets up
+  // kernel attributes and tensor maps. It counts as the first step of the flow,
+  // and where the floor detection may end an instance (between rounds, so after
+  // 1 + l K steps) both ways take it.
+  const bool lead = !direct || stall > 0;
+  if (lead)
     for (const auto &grp : groups) SPM_TRY(group_steps(ctx, phi, uh, grp, 1));
+  if (!direct) {
     e = cudaStreamBeginCapture(s0, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return spm_fail_cuda(e, "graph capture");
     advance();
@@ -144,7 +148,7 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
   }
   std::vector<int> host(8 * (size_t)n);
   std::vector<double> rec;
-  std::vector<int> seen(n, direct ? 0 : 1);  // (the step outside the graph is record 0)
+  std::vector<int> seen(n, lead ? 1 : 0);  // (the step ahead of the rounds is record 0)
   std::vector<FloorWatch> watch(n, FloorWatch(tol, stall > 0 ? stall : 1));
   static const int kZero = 0;
   const int launches = (max_steps + K - 1) / K;

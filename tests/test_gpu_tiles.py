@@ -105,3 +105,26 @@ def test_many_groups_run_through_a_graph(cuda):
     assert d0 == d1 == [70] * 9
     for a, b in zip(p0 + u0, p1 + u1):
         assert cuda.equal(a, b)
+
+
+@pytest.mark.parametrize("K", [16, 50])
+def test_floor_detection_does_not_depend_on_the_launch_path(cuda, K):
+    """Mixed batches whose FP32 phase ends at its rounding floor, between rounds of K
+    steps: launched directly (one group) or through the graph (nine), an instance
+    hands over to FP64 after the same step, with the same counts and fields."""
+    import spmiqc
+    out = []
+    for group in (0, 1):
+        cs = [spmiqc.SpmContext(32, L=18.0 + i, Tau=0.5 - 0.002 * i) for i in range(9)]
+        for c in cs:
+            c.tune("batch_group", group)
+        ps = [cuda.from_numpy(npo.uniform_field(32, 100 + i)).cuda() for i in range(9)]
+        us = [c.my_fft(p) for c, p in zip(cs, ps)]
+        cuda.cuda.synchronize()
+        out.append((spmiqc.batch_grad_flow(cs, ps, us, 12000, 1e-10, 1e-9, steps_per_launch=K), ps, us))
+        for c in cs:
+            c.close()
+    (d0, p0, u0), (d1, p1, u1) = out
+    assert d0 == d1
+    for a, b in zip(p0 + u0, p1 + u1):
+        assert cuda.equal(a, b)
