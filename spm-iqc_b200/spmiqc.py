@@ -547,7 +547,7 @@ def load_checkpoint(path: str):
 
 def batch_grad_flow(ctxs, phis, uhats, max_steps: int, tol_grad: float, switch_tol: float = 0.0,
                     steps_per_launch: int = 16):
-    """spm_batch_grad_flow: all instances advanced by one captured graph per launch; returns the steps per instance."""
+    """spm_batch_grad_flow: all instances advanced in rounds of steps_per_launch steps; returns the steps per instance."""
     n = len(ctxs)
     f = lib().spm_batch_grad_flow
     arr = ctypes.c_void_p * n
