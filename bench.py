@@ -372,7 +372,7 @@ def serve_ranks(specs, make_fields, rank, world, slots, precision_of, tol, fake=
 def batch_core(n_inst, cap, branches, rank=0, world=1):
     """Batched relaxations: n_inst instances of uneven sizes (N in {64, ...,
     256}, L ~ U[18, 30], Tau ~ U[-0.02, 0], BCC / FCC / icosahedral cosine
-    fields) relaxed together by spm_batch_grad_flow (one set of launches per
+    fields) relaxed together by spm_batch_grad_flow (one set of gated steps per
     launch; instances of one size share every launch; FP32 bulk, then FP64
     polish) to ||grad F|| <= 1e-8 or the step cap, next to the same instances
     relaxed one after another in FP64 with spm_grad_flow (the reference's one
