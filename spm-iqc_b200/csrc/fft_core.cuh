@@ -428,7 +428,8 @@ __device__ __forceinline__ float2 ld_keep(const float2 *p, uint64_t pol) {
 }
 
 // Streamed field data (read or written once per pass) with an L2 "evict
-// first" policy, so it does not push the exchange areas out of L2.
+// first" policy, so it does not push the exchange areas out of L2. Coherent
+// loads, as ld_field's: the launch before may be the writer.
 __device__ __forceinline__ uint64_t l2_stream_policy() {
   uint64_t pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -436,12 +437,12 @@ __device__ __forceinline__ uint64_t l2_stream_policy() {
 }
 __device__ __forceinline__ double2 ld_stream(const double2 *p, uint64_t pol) {
   double2 v;
-  asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ float2 ld_stream(const float2 *p, uint64_t pol) {
   float2 v;
-  asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
   return v;
 }
 // A value of a state spectrum that the same kernel overwrites (volatile, as the
@@ -468,6 +469,12 @@ __device__ __forceinline__ float2 ld_state(const float2 *p, uint64_t pol) {
   asm volatile("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
   return v;
 }
+// A value of a field that the launch before may have written. A kernel that is
+// launched early (grid_dep_sync) runs while that launch still writes, so the
+// field is not constant for its lifetime: a coherent load, kept behind the wait
+// (both volatile). __ldg is for data that is two launches old or older (the
+// launch before this one passed its own wait before this kernel started).
+template <class T2> __device__ __forceinline__ T2 ld_field(const T2 *p) { return ld_state(p); }
 __device__ __forceinline__ void st_stream(double2 *p, double2 v, uint64_t pol) { st_keep(p, v, pol); }
 __device__ __forceinline__ void st_stream(float2 *p, float2 v, uint64_t pol) { st_keep(p, v, pol); }
 
@@ -615,14 +622,16 @@ __device__ __forceinline__ bool flow_stopped(const KParams &p, int b) {
   const int *f = flow_of(p, b);
   return f != nullptr && *((volatile const int *)f + FW_GO) == 0;
 }
-// Both words in one load: returns flow_stopped, sets pending.
+// Both words in one load (volatile, as flow_stopped's, so that it stays behind
+// grid_dep_sync): returns flow_stopped, sets pending.
 __device__ __forceinline__ bool flow_state(const KParams &p, int b, bool &pending) {
   static_assert(FW_GO == 0 && FW_PENDING == 1, "one 8-byte load");
   const int *f = flow_of(p, b);
   if (f == nullptr) return false;
-  const int2 w = __ldcg(reinterpret_cast<const int2 *>(f));
-  pending = w.y != 0;
-  return w.x == 0;
+  int go, pend;
+  asm volatile("ld.volatile.global.v2.s32 {%0, %1}, [%2];" : "=r"(go), "=r"(pend) : "l"(f) : "memory");
+  pending = pend != 0;
+  return go == 0;
 }
 // The step's stop is armed (FW_PENDING, set by its pencil pass before launch).
 __device__ __forceinline__ bool flow_pending(const KParams &p, int b) {
@@ -665,6 +674,7 @@ __device__ __forceinline__ double fast_rcp(double x) {
 // by the cluster passes.
 struct SymFn {
   double g;
+  double pre;  // the scalar that an operator with PRE reads (pencil_kernel), else 0
   __device__ double G() const { return g; }
   __device__ double step(const ModelC &m) const { return fast_rcp(fma(m.dt, g, 1.0)); }  // 1/(1 + dt G)
   __device__ double prec(const ModelC &m) const { return fast_rcp(g + fabs(m.Tau) + 0.02); }

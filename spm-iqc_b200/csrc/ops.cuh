@@ -8,8 +8,10 @@ namespace spm {
 
 template <class T> __device__ __forceinline__ const T *fld(const void *p) { return reinterpret_cast<const T *>(p); }
 __device__ __forceinline__ double *scal_of(const KParams &p, int b) { return p.scal + (size_t)b * kScal; }
-// A scalar that an earlier kernel has written: constant here, so that a
-// thread's points share one load (and what is computed from it).
+// A scalar that the launch before last or an earlier one has written, for the
+// epilogues (their plane pass follows the pencil pass): constant for the
+// kernel's lifetime even if it is launched early, so that a thread's points share
+// one load (and what is computed from it).
 __device__ __forceinline__ double scal_in(const KParams &p, int b, int slot) {
   return __ldg(p.scal + (size_t)b * kScal + slot);
 }
@@ -72,7 +74,7 @@ template <class T> struct ProHv {
   static constexpr int NR = 2;
   static constexpr unsigned MAXM = 0;
   __device__ static c2<T> pro(const KParams &p, int b, size_t idx, c2<T> x, double (&acc)[2]) {
-    const c2<T> ph = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
+    const c2<T> ph = ld_field(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
     const T tau = (T)p.m.Tau, gam = (T)p.m.Gamma;
     acc[0] += (double)x.x + (double)x.y;
     acc[1] += (double)((-tau - (T)2 * gam * ph.x + (T)3 * ph.x * ph.x) * x.x);
@@ -128,8 +130,8 @@ template <class T> struct ProForce {
   static constexpr unsigned MAXM = 0;
   static constexpr bool FACC = true;
   template <class A> __device__ static c2<T> pro(const KParams &p, int b, size_t idx, c2<T> x, A (&acc)[4]) {
-    const c2<T> v = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
-    const c2<T> gv = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux1[b]) + idx));
+    const c2<T> v = ld_field(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
+    const c2<T> gv = ld_field(reinterpret_cast<const c2<T> *>(fld<T>(p.aux1[b]) + idx));
     const T tau = (T)p.m.Tau, gam = (T)p.m.Gamma;
     const T n0 = poly_force(x.x, tau, gam);
     const T n1 = poly_force(x.y, tau, gam);
@@ -154,7 +156,7 @@ template <class T> struct ProTangent {
   static constexpr unsigned MAXM = 0;
   static constexpr bool FACC = true;
   template <class A> __device__ static c2<T> pro(const KParams &p, int b, size_t idx, c2<T> x, A (&acc)[1]) {
-    const c2<T> a = p.aux0[b] ? __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx)) : c2<T>{0, 0};
+    const c2<T> a = p.aux0[b] ? ld_field(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx)) : c2<T>{0, 0};
     const c2<T> d = {x.x - a.x, x.y - a.y};
     acc[0] += (A)d.x * (A)d.x + (A)d.y * (A)d.y;
     return d;
@@ -172,7 +174,7 @@ template <class T> struct ProHisd {
   static constexpr int NR = 0;
   static constexpr unsigned MAXM = 0;
   __device__ static c2<T> pro(const KParams &p, int b, size_t idx, c2<T> x, double (&)[1]) {
-    const c2<T> t = __ldg(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
+    const c2<T> t = ld_field(reinterpret_cast<const c2<T> *>(fld<T>(p.aux0[b]) + idx));
     const T tau = (T)p.m.Tau, gam = (T)p.m.Gamma, beta = (T)p.m.factor;
     return c2<T>{x.x + beta * (poly_force(x.x, tau, gam) - t.x), x.y + beta * (poly_force(x.y, tau, gam) - t.y)};
   }
@@ -304,6 +306,7 @@ template <class T> struct OpPrecond {
 // with s = factor * <ngrad(x), v> from the prologue and v^ (st) the stored
 // spectrum of the tangent.
 template <class T> struct OpForce {
+  static constexpr int PRE = SC_S;  // written by the launch before
   static constexpr bool FI = true, SI = true, SO = false, INV = true, LIN = false;
   static constexpr bool SYM = true;
   static constexpr int NR = 0;
@@ -312,7 +315,7 @@ template <class T> struct OpForce {
   __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T> s, c2<T> &,
                                c2<T> &inv, double (&)[1], double) {
     const T iden = (T)sy.force();  // 1 / (1 + G)
-    const T sc = (T)scal_in(p, b, SC_S);
+    const T sc = (T)sy.pre;
     const c2<T> fh = cscale(f, (T)S::scale(p.m));
     inv = c2<T>{(fh.x - sc * s.x) * iden, (fh.y - sc * s.y) * iden};
     if (Kx == 0 && Ky == 0 && Kz == 0) inv = c2<T>{0, 0};
@@ -324,6 +327,7 @@ template <class T> struct OpForce {
 // field Gv = IFFT(G v^, k = 0 removed) (inverse output). With NORM false the
 // field is taken as given (||d|| := 1), for force steps along a caller's v.
 template <class T, bool NORM = true> struct OpTangent {
+  static constexpr int PRE = NORM ? SC_NRM2 : -1;  // written by the launch before
   static constexpr bool FI = true, SI = false, SO = true, INV = true, LIN = false;
   static constexpr bool SYM = true;
   static constexpr int NR = 0;
@@ -331,7 +335,7 @@ template <class T, bool NORM = true> struct OpTangent {
   template <class S>
   __device__ static void point(const KParams &p, int b, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T>, c2<T> &so,
                                c2<T> &inv, double (&)[1], double) {
-    const T inrm = NORM ? (T)(1.0 / sqrt(scal_in(p, b, SC_NRM2))) : (T)1;
+    const T inrm = NORM ? (T)(1.0 / sqrt(sy.pre)) : (T)1;
     const c2<T> v = cscale(cscale(f, (T)S::scale(p.m)), inrm);
     so = v;
     inv = (Kx == 0 && Ky == 0 && Kz == 0) ? c2<T>{0, 0} : cscale(v, (T)sy.G());

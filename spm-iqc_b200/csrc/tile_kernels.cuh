@@ -349,6 +349,11 @@ template <int N, class T> struct Plane {
 template <class X, class = void> struct AuxOf : std::integral_constant<int, 0> {};
 template <class X> struct AuxOf<X, std::void_t<decltype(X::AUX)>> : std::integral_constant<int, X::AUX> {};
 
+// The slot of the scalar block that an operator needs from the launch before: X::PRE,
+// else none (-1).
+template <class X, class = void> struct PreOf : std::integral_constant<int, -1> {};
+template <class X> struct PreOf<X, std::void_t<decltype(X::PRE)>> : std::integral_constant<int, X::PRE> {};
+
 // Asks for the 32 rows of tile (x, j2) of a real field to be brought into L2 (one
 // warp; bulk prefetches want 16-byte alignment, which FP32 fields need not have).
 // From 96^3 to 192^3 only (Hessian products in blocks of 8, FP64, without and
@@ -495,7 +500,7 @@ __global__ void __launch_bounds__(N, PlaneGeo<N, T>::CPS)
       const size_t off = ((size_t)x * N + YB * r + j2) * N;
       const T2 *row = reinterpret_cast<const T2 *>(src + off);
       T2 v[N1];
-      sfor<0, N1>([&](auto J) { v[SPM_CI(J)] = __ldg(row + 8 * SPM_CI(J) + jz); });
+      sfor<0, N1>([&](auto J) { v[SPM_CI(J)] = ld_field(row + 8 * SPM_CI(J) + jz); });
       run_prologue<T, Pro, N1>(
           [&](auto &a) {
             sfor<0, N1>([&](auto J) {
@@ -710,6 +715,9 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
   grid_dep_sync();
   if (p.trigger) grid_dep_trigger();
   if (flow_stopped(p, field_id())) return;
+  // read once, behind the wait (volatile): a register for all points
+  double pre = 0.0;
+  if constexpr (PreOf<Op>::value >= 0) pre = *((volatile const double *)p.scal + b * kScal + PreOf<Op>::value);
   const int cc = tid % C;
   const int jx = (tid / C) % M1, j2 = tid / (M1 * C);  // first / last phase
   const bool has_io = j2 < YB;
@@ -782,7 +790,7 @@ __global__ void __launch_bounds__(PencilGeo<N, T>::TH, PencilGeo<N, T>::CPS)
       const double2 gy = gx[Ky < 0 ? -Ky : Ky], gz = gx[col];
       gyz = double2{gy.x * gz.x, gy.y + gz.y};
     }
-    auto sym = [&](int Kx, double2 yz) { return SymFn{Op::SYM ? pair_symbol(gx[Kx < 0 ? -Kx : Kx], yz) : 0.0}; };
+    auto sym = [&](int Kx, double2 yz) { return SymFn{Op::SYM ? pair_symbol(gx[Kx < 0 ? -Kx : Kx], yz) : 0.0, pre}; };
     const bool packed = !Op::LIN && col == 0;
     constexpr int SG = M1 <= 8 ? M1 : M1 / 2;  // state loads in flight per thread
     constexpr bool STREAM = stream_state<N, T>();

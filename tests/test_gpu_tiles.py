@@ -128,3 +128,43 @@ def test_floor_detection_does_not_depend_on_the_launch_path(cuda, K):
     assert d0 == d1
     for a, b in zip(p0 + u0, p1 + u1):
         assert cuda.equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("N", [32, 64, 128])
+def test_operations_in_a_row_read_what_the_one_before_wrote(cuda, N, prec):
+    """Grids of one wave are launched while the launch before still runs. Operations
+    in a row, each on the fields that the one before has just written (tangent,
+    force steps along it, a Hessian product, a preconditioner, transforms and a
+    flow), give the same bits as with the device idle in between."""
+    import spmiqc
+    dt = np.float64 if prec == "fp64" else np.float32
+    c = spmiqc.SpmContext(N, Tau=-0.02, precision=prec)
+    a, b = (cuda.from_numpy(npo.uniform_field(N, s).astype(dt)).cuda() for s in (3, 4))
+    out = []
+    for idle in (False, True):
+        got = []
+
+        def did(x):
+            got.append(x)
+            if idle:
+                cuda.cuda.synchronize()
+            return x
+
+        x = did(a.clone())
+        for _ in range(4):
+            v = did(c.get_Tv(x, b))
+            did(c.Natural_Forces(x, v))
+            did(c.MinMax_Forces(x, v))
+            h = did(c.hv_cam(x, v))
+            did(c.precond_camnew(h))
+            x = did(x + 0.01 * h)  # small: the flow below stays stable
+            did(c.get_Tv(v, x, h))
+            u = did(c.my_fft(x))
+            did(c.my_ifft(u, x))
+            c.get_min_u_F(x, u, 3)
+        cuda.cuda.synchronize()
+        out.append([t.clone() for t in got])
+    for p, q in zip(*out):
+        assert cuda.equal(p, q)
+    c.close()
