@@ -113,13 +113,19 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s0, st.ev[g], 0);
     }
   };
-  // Up to kDirectGroups groups are launched step by step: two launches a step
-  // and group take the host less time than the device needs for the step, and a
-  // graph costs its capture and instantiation first (2 ms for three groups of
-  // 16 steps, against 85 us a step on the device). Many groups (instances
-  // that share no launch) go through a captured graph of K steps.
+  // A graph of K steps costs its capture and instantiation first (0.7 ms for one
+  // group at K = 16, 1.2-1.6 for two or three, 2-4 for four to eight); launching
+  // the steps directly costs the host about 4 us a launch, all groups from one
+  // thread, where the graph's branches overlap. So long runs take the graph, the
+  // sooner the more groups there are, judged by the rounds that max_steps
+  // allows. us a step, direct / graph: eight 32^3 instances 120 / 128 over 2 rounds,
+  // 73 / 46 over 8, 62 / 25 over 128; four 44 / 31 over 8; two 27 / 24 over 8, 24 / 17 over
+  // 128; groups of 64^3, 96^3, 128^3 118 / 133 over 2, 103 / 101 over 8, 98 / 93 over 128. One
+  // group keeps the device busy either way: 18 / 20 over 8 rounds, 16.6 / 16.0 over 32.
+  // More than kDirectGroups groups take the graph at any length.
   constexpr int kDirectGroups = 8;
-  const bool direct = ng <= kDirectGroups;
+  const int launches = (max_steps + K - 1) / K;  // rounds at most
+  const bool direct = ng <= kDirectGroups && (ng == 1 ? launches < 32 : launches < (24 + ng - 1) / ng);
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   for (int i = 0; i < n; i++) ctx[i]->stream = s0;
@@ -151,7 +157,6 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
   std::vector<int> seen(n, lead ? 1 : 0);  // (the step ahead of the rounds is record 0)
   std::vector<FloorWatch> watch(n, FloorWatch(tol, stall > 0 ? stall : 1));
   static const int kZero = 0;
-  const int launches = (max_steps + K - 1) / K;
   for (int l = 0; l < launches && rc == SPM_OK; l++) {
     if (direct) advance();
     else e = cudaGraphLaunch(exec, s0);

@@ -168,3 +168,33 @@ def test_operations_in_a_row_read_what_the_one_before_wrote(cuda, N, prec):
     for p, q in zip(*out):
         assert cuda.equal(p, q)
     c.close()
+
+
+@pytest.mark.parametrize("ng,steps,graph", [(2, 176, False), (2, 192, True), (8, 32, False), (8, 48, True),
+                                            (1, 496, False), (1, 512, True)])
+def test_long_batches_of_several_groups_take_the_graph(cuda, ng, steps, graph):
+    """Groups that share no launch (batch_group 0) are launched from one host thread:
+    over 24 / ng rounds or more (32 for one group) they go through the captured graph, whose
+    launches the host issues once. The host's launches tell the ways apart (a step takes two,
+    a captured one is counted once), and fields and counts are those of a plain flow."""
+    import spmiqc
+    K = 16
+    cs = [spmiqc.SpmContext(32, L=18.0 + i) for i in range(ng)]
+    for c in cs:
+        c.tune("batch_group", 0)
+    start = [npo.uniform_field(32, 200 + i) for i in range(ng)]
+    ps = [cuda.from_numpy(x.copy()).cuda() for x in start]
+    us = [c.my_fft(p) for c, p in zip(cs, ps)]
+    cuda.cuda.synchronize()
+    count = spmiqc.lib().spm_launch_count
+    before = [count(c.h) for c in cs]
+    assert spmiqc.batch_grad_flow(cs, ps, us, steps, 1e-14, steps_per_launch=K) == [steps] * ng
+    for c, b in zip(cs, before):
+        # one step ahead and one captured round, or every round
+        assert (count(c.h) - b < 4 * K) == graph
+    for c, x, p, u in zip(cs, start, ps, us):
+        q = cuda.from_numpy(x).cuda()
+        w = c.my_fft(q)
+        c.get_min_u_F(q, w, steps)
+        assert cuda.equal(p, q) and cuda.equal(u, w)
+        c.close()
