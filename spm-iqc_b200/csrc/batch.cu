@@ -41,6 +41,28 @@ struct Streams {
   }
 };
 
+// The contexts of a phase run on its streams and carry its limits; on every way
+// out they get their own stream back and carry none, and no work of a failed
+// phase stays in flight on streams that go away.
+struct Bound {
+  spm_ctx *const *ctx;
+  const Streams &st;
+  std::vector<cudaStream_t> saved;
+  bool done = false;  // the phase ended with its streams idle
+  Bound(spm_ctx *const *c, int n, const Streams &s) : ctx(c), st(s) {
+    for (int i = 0; i < n; i++) saved.push_back(c[i]->stream);
+  }
+  ~Bound() {
+    if (!done)
+      for (cudaStream_t x : st.s) cudaStreamSynchronize(x);
+    for (size_t i = 0; i < saved.size(); i++) {
+      ctx[i]->stream = saved[i];
+      ctx[i]->m.tol_grad = 0.0;
+      ctx[i]->m.max_steps = 0.0;
+    }
+  }
+};
+
 // Instances grouped by (N, precision), at most kMaxBatch per group, in order
 // of first appearance; with `group` false every instance is its own group.
 std::vector<std::vector<int>> make_groups(spm_ctx *const *ctx, int n, bool group) {
@@ -90,10 +112,9 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
       return spm_fail(SPM_ERR_CUDA, "batch streams");
   }
   cudaStream_t s0 = st.s[ng];
-  std::vector<cudaStream_t> saved(n);
+  Bound bound(ctx, n, st);
   for (int i = 0; i < n; i++) {
-    saved[i] = ctx[i]->stream;
-    cudaStreamSynchronize(saved[i]);  // earlier work of the instance is complete
+    cudaStreamSynchronize(bound.saved[i]);  // earlier work of the instance is complete
     SPM_TRY(spm_ensure_scratch(ctx[i], 1));
     SPM_TRY(spm_ensure_stats(ctx[i], max_steps + K));
     SPM_TRY(spm_flow_init(ctx[i], s0));
@@ -203,16 +224,12 @@ int run_phase(spm_ctx *const *ctx, void *const *phi, void *const *uh, int n, int
     }
     if (all || rc != SPM_OK) break;
   }
-  if (rc != SPM_OK)  // nothing of a failed round stays in flight
+  if (rc != SPM_OK)  // (a graph in flight is not destroyed)
     for (cudaStream_t x : st.s) cudaStreamSynchronize(x);
   if (exec) cudaGraphExecDestroy(exec);
   if (graph) cudaGraphDestroy(graph);
-  for (int i = 0; i < n; i++) {
-    ctx[i]->stream = saved[i];
-    ctx[i]->m.tol_grad = 0.0;
-    ctx[i]->m.max_steps = 0.0;
-    steps[i] += host[8 * (size_t)i + FW_ITER];
-  }
+  for (int i = 0; i < n; i++) steps[i] += host[8 * (size_t)i + FW_ITER];
+  bound.done = true;
   return rc;
 }
 

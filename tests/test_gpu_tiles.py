@@ -198,3 +198,30 @@ def test_long_batches_of_several_groups_take_the_graph(cuda, ng, steps, graph):
         c.get_min_u_F(q, w, steps)
         assert cuda.equal(p, q) and cuda.equal(u, w)
         c.close()
+
+
+@pytest.mark.parametrize("n", [2, 9])
+def test_refused_batch_gives_its_contexts_back(cuda, n):
+    """A batch whose last spectrum is not 16-byte aligned is refused after its streams
+    exist, launched directly (2 groups) or on the way to the graph (9): the contexts
+    run on their own stream again, without the batch's limits."""
+    import spmiqc
+    N = 32
+    cs = [spmiqc.SpmContext(N, L=18.0 + i) for i in range(n)]
+    for c in cs:
+        c.tune("batch_group", 0)
+    start = [npo.uniform_field(N, 300 + i) for i in range(n)]
+    ps = [cuda.from_numpy(x.copy()).cuda() for x in start]
+    us = [c.my_fft(p) for c, p in zip(cs, ps)]
+    odd = cuda.zeros(N ** 3 + 1, dtype=cuda.float64, device="cuda")[1:]
+    cuda.cuda.synchronize()
+    with pytest.raises(spmiqc.SpmError) as err:
+        spmiqc.batch_grad_flow(cs, ps, us[:-1] + [odd], 64, 1e30)
+    assert err.value.status == spmiqc.SPM_ERR_ARG
+    for c, x in zip(cs, start):
+        m = npo.Model(N, L=c.L)
+        q = cuda.from_numpy(x.copy()).cuda()
+        u = c.my_fft(q)
+        assert rel(c.to_full(u).cpu().numpy(), m.my_fft(x)) < 1e-11
+        assert len(c.get_min_u_F(q, u, 5)) == 5
+        c.close()
