@@ -122,8 +122,8 @@ const char *spm_status_str(int status);
 int spm_tune(spm_ctx *ctx, const char *knob, int value);
 int spm_tune_get(const spm_ctx *ctx, const char *knob);
 /* Autotuner (no counterpart in the reference): times chains of `steps`
- * gradient steps on a scratch field for each candidate schedule (FP64: pdl 0
- * and 1; FP32: plane_cps 1/2/3 with fused chains, plane_cps 2 without, plane_xg 1/2/3 with plane_cps
+ * gradient steps on a scratch field for each candidate schedule (FP64: fused
+ * chains, without, then pdl 1; FP32: plane_cps 1/2/3 with fused chains, plane_cps 2 without, plane_xg 1/2/3 with plane_cps
  * 2 and 3 on fused chains, plane_cps 4 for FP32, 5, 6; then pencil_tc 4 and
  * pdl 1 for the best of them), keeping a later candidate only if it is at least 1 % faster, and
  * keeps the fastest in the context; the choice is remembered per (device, N, precision), so later

@@ -1,9 +1,10 @@
 // Autotuner for the transform schedule of a context (no counterpart in the
 // reference; FFTW's plan search plays this role there, My_FFT.cpp:49-97).
-// FP64 contexts (tile passes): programmatic dependent launches or not (knob
-// "pdl"). FP32 contexts (cluster passes): the plane-pass variant (staged with one CTA per SM, direct loads
+// FP64 contexts (tile passes): whether gradient chains use the fused inverse ->
+// forward plane pass, and programmatic dependent launches or not (knob "pdl").
+// FP32 contexts (cluster passes): the plane-pass variant (staged with one CTA per SM, direct loads
 // with two CTAs per SM, or three CTAs per SM with fewer registers per thread),
-// whether gradient chains use the fused inverse -> forward plane pass, and
+// the fused plane pass or not, and
 // whether their plane kernels exchange through distributed shared memory or
 // through global areas resident in L2; then, for the fastest, the pencil tile
 // width and programmatic dependent launches (knob "pdl").
@@ -58,12 +59,18 @@ bool spm_autotune_lookup(int device, int N, int prec, int *plane_cps, int *fuse_
 extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_planes) {
   if (!c || steps < 2) return spm_fail(SPM_ERR_ARG, "bad argument (steps >= 2)");
   const auto key = std::make_tuple(c->device, c->N, c->prec);
-  auto finish = [&](const Choice &ch) {
-    c->plane_cps = ch.plane_cps;
+  // The knobs that concern the context's kernels: an FP64 one keeps those that
+  // only its FP32 twin reads.
+  auto apply = [&](const Choice &ch) {
     c->fuse_planes = ch.fuse_planes;
+    c->pdl = ch.pdl;
+    if (c->prec == SPM_FP64) return;
+    c->plane_cps = ch.plane_cps;
     c->plane_xg = ch.plane_xg;
     c->pencil_tc = ch.pencil_tc;
-    c->pdl = ch.pdl;
+  };
+  auto finish = [&](const Choice &ch) {
+    apply(ch);
     if (!c->plane_xg && c->xg) {  // the exchange areas are not used by the chosen schedule
       cudaStreamSynchronize(c->stream);
       cudaFree(c->xg);
@@ -96,8 +103,9 @@ extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_pla
   const Choice cands[] = {{2, 1, 0}, {3, 1, 0}, {1, 1, 0}, {2, 0, 0}, {2, 1, spm::kXgFwd | spm::kXgInv},
                           {3, 1, spm::kXgFwd | spm::kXgInv}, {2, 1, spm::kXgFwd}, {2, 1, spm::kXgInv}};
   std::vector<Choice> all(std::begin(cands), std::end(cands));
-  // FP64 chains run on the tile passes, which only "pdl" concerns
-  if (c->prec == SPM_FP64) all.assign(1, Choice{c->plane_cps, c->fuse_planes, c->plane_xg, c->pencil_tc});
+  // FP64 chains run on the tile passes, without variants of the planes (the list
+  // does not depend on the context: the choice serves later ones too)
+  if (c->prec == SPM_FP64) all = {{2, 1, 0}, {2, 0, 0}};
   if (c->prec == SPM_FP32) all.push_back({4, 1, spm::kXgFwd | spm::kXgInv});  // four CTAs per SM
   if (c->prec == SPM_FP32) {
     all.push_back({5, 1, spm::kXgFwd | spm::kXgInv});  // 16-row CTAs, four per SM
@@ -105,11 +113,7 @@ extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_pla
   }
   // best of three timed chains of `steps` gated steps with the candidate's knobs
   auto time_it = [&](const Choice &cand, float &t) -> int {
-    c->plane_cps = cand.plane_cps;
-    c->fuse_planes = cand.fuse_planes;
-    c->plane_xg = cand.plane_xg;
-    c->pencil_tc = cand.pencil_tc;
-    c->pdl = cand.pdl;
+    apply(cand);
     int r = spm_ensure_xg(c);
     if (r != SPM_OK) return r;
     if (c->prec == SPM_FP64) fill_kernel<double><<<592, 256, 0, c->stream>>>((double *)phi, c->N);

@@ -225,3 +225,22 @@ def test_refused_batch_gives_its_contexts_back(cuda, n):
         assert rel(c.to_full(u).cpu().numpy(), m.my_fft(x)) < 1e-11
         assert len(c.get_min_u_F(q, u, 5)) == 5
         c.close()
+
+
+def test_autotuned_choice_does_not_depend_on_the_first_context(cuda):
+    """The remembered FP64 choice comes from fixed candidates: a first context with
+    the fused plane pass off (a store and a load of phi more a step) does not switch it
+    off for later ones. The knobs that FP64 kernels do not read stay the caller's."""
+    import spmiqc
+    N = 160
+    c = spmiqc.SpmContext(N)
+    c.tune("fuse_planes", 0)
+    c.tune("plane_cps", 3)
+    c.autotune(20)
+    assert c.tuning()["fuse_planes"] == 1 and c.tuning()["plane_cps"] == 3
+    d = spmiqc.SpmContext(N)
+    d.autotune(20)
+    assert d.tuning()["fuse_planes"] == 1 and d.tuning()["plane_cps"] == 2
+    assert d.tuning()["pdl"] == c.tuning()["pdl"]
+    c.close()
+    d.close()
