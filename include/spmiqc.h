@@ -118,7 +118,10 @@ const char *spm_status_str(int status);
  * completes, and its kernel waits on the device for that kernel before its
  * first memory access; 0 (default) = plain stream order. The same bits
  * either way; spm_autotune turns it on where it is at least 1 % faster.
- * spm_tune_get returns the current value or -1 for an unknown knob. */
+ * spm_tune_get returns the current value or -1 for an unknown knob; on FP64
+ * contexts "twin_" before a name (twin_plane_cps, twin_fuse_planes, twin_plane_xg,
+ * twin_pencil_tc, twin_pdl) gives what the FP32 twin of mixed runs takes: the
+ * context's own knobs, or the autotuner's choice for the twin if they were not set since. */
 int spm_tune(spm_ctx *ctx, const char *knob, int value);
 int spm_tune_get(const spm_ctx *ctx, const char *knob);
 /* Autotuner (no counterpart in the reference): times chains of `steps`
@@ -128,7 +131,8 @@ int spm_tune_get(const spm_ctx *ctx, const char *knob);
  * pdl 1 for the best of them), keeping a later candidate only if it is at least 1 % faster, and
  * keeps the fastest in the context; the choice is remembered per (device, N, precision), so later
  * contexts of the same kind take it without timing (FP32 twins of mixed flows
- * included). Synchronises; allocates two scratch fields while it runs. The
+ * included). On an FP64 context it also chooses the FP32 schedule of its twin, by the same
+ * search on an FP32 context that it makes for the purpose. Synchronises; allocates two scratch fields while it runs. The
  * chosen knobs are returned in *plane_cps, *fuse_planes (may be NULL);
  * spm_tune_get(ctx, "plane_xg") gives the exchange route. */
 int spm_autotune(spm_ctx *ctx, int steps, int *plane_cps, int *fuse_planes);

@@ -8,6 +8,7 @@
 // whether their plane kernels exchange through distributed shared memory or
 // through global areas resident in L2; then, for the fastest, the pencil tile
 // width and programmatic dependent launches (knob "pdl").
+// Tuning an FP64 context also chooses the FP32 schedule of its twin (mixed flows).
 // Each candidate runs a short chain of gradient steps on a scratch field with
 // CUDA events around it; the fastest is kept in the context and remembered per
 // (device, N, precision) for later contexts.
@@ -28,6 +29,7 @@ struct Choice {
   int plane_cps, fuse_planes, plane_xg, pencil_tc = 8, pdl = 0;
 };
 std::map<std::tuple<int, int, int>, Choice> g_best;  // (device, N, prec) -> schedule
+std::map<std::tuple<int, int, int>, Choice> g_twin;  // the same for twins of tuned FP64 contexts
 
 // A smooth non-trivial field (a few cosines), so the timed steps do real work
 // and the flow does not stop on its first step.
@@ -40,55 +42,19 @@ template <class T> __global__ void fill_kernel(T *phi, int N) {
   }
 }
 
-}  // namespace
-
-// The remembered choice for (device, N, precision), if any.
-bool spm_autotune_lookup(int device, int N, int prec, int *plane_cps, int *fuse_planes, int *plane_xg,
-                         int *pencil_tc, int *pdl) {
-  std::lock_guard<std::mutex> lk(g_mu);
-  auto it = g_best.find(std::make_tuple(device, N, prec));
-  if (it == g_best.end()) return false;
-  *plane_cps = it->second.plane_cps;
-  *fuse_planes = it->second.fuse_planes;
-  *plane_xg = it->second.plane_xg;
-  if (pencil_tc) *pencil_tc = it->second.pencil_tc;
-  if (pdl) *pdl = it->second.pdl;
-  return true;
+// The knobs that concern the context's kernels: an FP64 one keeps those that
+// only its FP32 twin reads.
+void apply(spm_ctx *c, const Choice &ch) {
+  c->fuse_planes = ch.fuse_planes;
+  c->pdl = ch.pdl;
+  if (c->prec == SPM_FP64) return;
+  c->plane_cps = ch.plane_cps;
+  c->plane_xg = ch.plane_xg;
+  c->pencil_tc = ch.pencil_tc;
 }
 
-extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_planes) {
-  if (!c || steps < 2) return spm_fail(SPM_ERR_ARG, "bad argument (steps >= 2)");
-  const auto key = std::make_tuple(c->device, c->N, c->prec);
-  // The knobs that concern the context's kernels: an FP64 one keeps those that
-  // only its FP32 twin reads.
-  auto apply = [&](const Choice &ch) {
-    c->fuse_planes = ch.fuse_planes;
-    c->pdl = ch.pdl;
-    if (c->prec == SPM_FP64) return;
-    c->plane_cps = ch.plane_cps;
-    c->plane_xg = ch.plane_xg;
-    c->pencil_tc = ch.pencil_tc;
-  };
-  auto finish = [&](const Choice &ch) {
-    apply(ch);
-    if (!c->plane_xg && c->xg) {  // the exchange areas are not used by the chosen schedule
-      cudaStreamSynchronize(c->stream);
-      cudaFree(c->xg);
-      c->xg = nullptr;
-      c->xg_cap = 0;
-    }
-    if (plane_cps) *plane_cps = c->plane_cps;
-    if (fuse_planes) *fuse_planes = c->fuse_planes;
-    return spm_ensure_xg(c);
-  };
-  {
-    std::lock_guard<std::mutex> lk(g_mu);
-    auto it = g_best.find(key);
-    if (it != g_best.end()) {
-      const Choice ch = it->second;
-      return finish(ch);
-    }
-  }
+// Times the candidates on the context; leaves its knobs changed.
+int search(spm_ctx *c, int steps, Choice *out) {
   void *phi = nullptr, *uh = nullptr;
   cudaError_t e = cudaMalloc(&phi, c->field_bytes);
   if (e == cudaSuccess) e = cudaMalloc(&uh, c->field_bytes);
@@ -96,8 +62,7 @@ extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_pla
   if (e == cudaSuccess) e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   int rc = e == cudaSuccess ? SPM_OK : spm_fail_cuda(e, "autotune buffers");
-  const Choice saved = {c->plane_cps, c->fuse_planes, c->plane_xg, c->pencil_tc, c->pdl};
-  Choice best = saved;
+  Choice best = {c->plane_cps, c->fuse_planes, c->plane_xg, c->pencil_tc, c->pdl};
   float best_ms = 1e30f;
   // plane variant, fused plane pass, exchange routes of the gradient chains
   const Choice cands[] = {{2, 1, 0}, {3, 1, 0}, {1, 1, 0}, {2, 0, 0}, {2, 1, spm::kXgFwd | spm::kXgInv},
@@ -113,7 +78,7 @@ extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_pla
   }
   // best of three timed chains of `steps` gated steps with the candidate's knobs
   auto time_it = [&](const Choice &cand, float &t) -> int {
-    apply(cand);
+    apply(c, cand);
     int r = spm_ensure_xg(c);
     if (r != SPM_OK) return r;
     if (c->prec == SPM_FP64) fill_kernel<double><<<592, 256, 0, c->stream>>>((double *)phi, c->N);
@@ -172,13 +137,101 @@ extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_pla
   if (e1) cudaEventDestroy(e1);
   cudaFree(phi);
   cudaFree(uh);
-  if (rc != SPM_OK) {
-    finish(saved);
-    return rc;
-  }
+  if (rc == SPM_OK) *out = best;
+  return rc;
+}
+
+// The schedule of an FP64 context's FP32 twin: what an FP32 context of the size
+// has been tuned to, else the fastest on a context made for the search. Without
+// room for that one the twin keeps the FP64 context's knobs.
+void tune_twin(spm_ctx *c, int steps) {
+  const auto key = std::make_tuple(c->device, c->N, (int)SPM_FP32);
+  Choice ch;
+  bool known = false;
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    g_best[key] = best;
+    for (auto *m : {&g_best, &g_twin}) {
+      auto it = m->find(key);
+      if (known || it == m->end()) continue;
+      ch = it->second;
+      known = true;
+    }
   }
-  return finish(best);
+  if (!known) {
+    spm_ctx *t = nullptr;
+    int rc = spm_ctx_create(c->N, c->L, c->m.Tau, c->m.Gamma, c->m.dt, SPM_FP32, c->stream, &t);
+    if (rc == SPM_OK) rc = search(t, steps, &ch);
+    if (t) spm_ctx_destroy(t);
+    if (rc != SPM_OK) {
+      cudaGetLastError();  // a refused allocation
+      return;
+    }
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_twin[key] = ch;
+  }
+  c->twin_plane_cps = ch.plane_cps;
+  c->twin_fuse_planes = ch.fuse_planes;
+  c->twin_plane_xg = ch.plane_xg;
+  c->twin_pencil_tc = ch.pencil_tc;
+  c->twin_pdl = ch.pdl;
+  c->twin_tuned = true;
+}
+
+}  // namespace
+
+// The remembered choice for (device, N, precision), if any.
+bool spm_autotune_lookup(int device, int N, int prec, int *plane_cps, int *fuse_planes, int *plane_xg,
+                         int *pencil_tc, int *pdl) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  auto it = g_best.find(std::make_tuple(device, N, prec));
+  if (it == g_best.end()) return false;
+  *plane_cps = it->second.plane_cps;
+  *fuse_planes = it->second.fuse_planes;
+  *plane_xg = it->second.plane_xg;
+  if (pencil_tc) *pencil_tc = it->second.pencil_tc;
+  if (pdl) *pdl = it->second.pdl;
+  return true;
+}
+
+extern "C" int spm_autotune(spm_ctx *c, int steps, int *plane_cps, int *fuse_planes) {
+  if (!c || steps < 2) return spm_fail(SPM_ERR_ARG, "bad argument (steps >= 2)");
+  const auto key = std::make_tuple(c->device, c->N, c->prec);
+  auto finish = [&](const Choice &ch) {
+    apply(c, ch);
+    if (!c->plane_xg && c->xg) {  // the exchange areas are not used by the chosen schedule
+      cudaStreamSynchronize(c->stream);
+      cudaFree(c->xg);
+      c->xg = nullptr;
+      c->xg_cap = 0;
+    }
+    if (plane_cps) *plane_cps = c->plane_cps;
+    if (fuse_planes) *fuse_planes = c->fuse_planes;
+    return spm_ensure_xg(c);
+  };
+  Choice ch;
+  bool known = false;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_best.find(key);
+    if (it != g_best.end()) {
+      ch = it->second;
+      known = true;
+    } else if (auto tw = g_twin.find(key); tw != g_twin.end()) {  // (FP32) searched for a twin before
+      ch = g_best[key] = tw->second;
+      known = true;
+    }
+  }
+  if (!known) {
+    const Choice saved = {c->plane_cps, c->fuse_planes, c->plane_xg, c->pencil_tc, c->pdl};
+    const int rc = search(c, steps, &ch);
+    if (rc != SPM_OK) {
+      finish(saved);
+      return rc;
+    }
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_best[key] = ch;
+  }
+  const int rc = finish(ch);
+  if (rc == SPM_OK && c->prec == SPM_FP64) tune_twin(c, steps);
+  return rc;
 }

@@ -414,21 +414,37 @@ extern "C" int spm_ctx_destroy(spm_ctx *c) {
   return SPM_OK;
 }
 
+// The schedule of the context's FP32 twin: its own knobs, or what spm_autotune
+// chose for the twin since they were last set; an FP32 schedule chosen by spm_autotune
+// on an FP32 context of this size wins.
+static void twin_schedule(const spm_ctx *c, int *plane_cps, int *fuse_planes, int *plane_xg, int *pencil_tc, int *pdl) {
+  const bool t = c->twin_tuned;
+  *plane_cps = t ? c->twin_plane_cps : c->plane_cps;
+  *fuse_planes = t ? c->twin_fuse_planes : c->fuse_planes;
+  *plane_xg = t ? c->twin_plane_xg : c->plane_xg;
+  *pencil_tc = t ? c->twin_pencil_tc : c->pencil_tc;
+  *pdl = t ? c->twin_pdl : c->pdl;
+  spm_autotune_lookup(c->device, c->N, SPM_FP32, plane_cps, fuse_planes, plane_xg, pencil_tc, pdl);
+}
+
 extern "C" int spm_tune(spm_ctx *c, const char *knob, int value) {
   if (!c || !knob) return spm_fail(SPM_ERR_ARG, "null argument");
   if (std::strcmp(knob, "plane_cps") == 0) {
     if (value < 1 || value > 6) return spm_fail(SPM_ERR_ARG, "plane_cps must be 1 to 6");
     c->plane_cps = value;
+    c->twin_tuned = false;
     return SPM_OK;
   }
   if (std::strcmp(knob, "fuse_planes") == 0) {
     if (value != 0 && value != 1) return spm_fail(SPM_ERR_ARG, "fuse_planes must be 0 or 1");
     c->fuse_planes = value;
+    c->twin_tuned = false;
     return SPM_OK;
   }
   if (std::strcmp(knob, "plane_xg") == 0) {
     if (value < 0 || value > 3) return spm_fail(SPM_ERR_ARG, "plane_xg must be 0..3");
     c->plane_xg = value;
+    c->twin_tuned = false;
     return spm_ensure_xg(c);
   }
   if (std::strcmp(knob, "batch_group") == 0) {
@@ -439,6 +455,7 @@ extern "C" int spm_tune(spm_ctx *c, const char *knob, int value) {
   if (std::strcmp(knob, "pencil_tc") == 0) {
     if (value != 8 && value != 4) return spm_fail(SPM_ERR_ARG, "pencil_tc must be 8 or 4");
     c->pencil_tc = value;
+    c->twin_tuned = false;
     return SPM_OK;
   }
   if (std::strcmp(knob, "block_stage") == 0) {
@@ -449,6 +466,7 @@ extern "C" int spm_tune(spm_ctx *c, const char *knob, int value) {
   if (std::strcmp(knob, "pdl") == 0) {
     if (value != 0 && value != 1) return spm_fail(SPM_ERR_ARG, "pdl must be 0 or 1");
     c->pdl = value;
+    c->twin_tuned = false;
     return SPM_OK;
   }
   return spm_fail(SPM_ERR_ARG, "unknown tuning knob");
@@ -463,6 +481,13 @@ extern "C" int spm_tune_get(const spm_ctx *c, const char *knob) {
   if (std::strcmp(knob, "pencil_tc") == 0) return c->pencil_tc;
   if (std::strcmp(knob, "block_stage") == 0) return c->block_stage;
   if (std::strcmp(knob, "pdl") == 0) return c->pdl;
+  if (c->prec == SPM_FP64 && std::strncmp(knob, "twin_", 5) == 0) {
+    static const char *const names[] = {"plane_cps", "fuse_planes", "plane_xg", "pencil_tc", "pdl"};
+    int v[5];
+    twin_schedule(c, &v[0], &v[1], &v[2], &v[3], &v[4]);
+    for (int i = 0; i < 5; i++)
+      if (std::strcmp(knob + 5, names[i]) == 0) return v[i];
+  }
   return -1;
 }
 
@@ -658,25 +683,19 @@ bool FloorWatch::step(double r) {
 }
 
 int spm_ensure_twin(spm_ctx *c) {
-  if (!c->twin) {
+  if (!c->twin) SPM_TRY(spm_ctx_create(c->N, c->L, c->m.Tau, c->m.Gamma, c->m.dt, SPM_FP32, c->stream, &c->twin));
+  if (!c->twin_buf) {
     const size_t n = (size_t)c->N * c->N * c->N;
-    SPM_TRY(spm_ctx_create(c->N, c->L, c->m.Tau, c->m.Gamma, c->m.dt, SPM_FP32, c->stream, &c->twin));
     cudaError_t e = cudaMalloc(&c->twin_buf, 2 * n * sizeof(float));
     if (e != cudaSuccess) return spm_fail_cuda(e, "FP32 twin fields");
   }
   c->twin->stream = c->stream;
   c->twin->cancel = c->cancel;
-  c->twin->plane_cps = c->plane_cps;
-  c->twin->fuse_planes = c->fuse_planes;
-  c->twin->plane_xg = c->plane_xg;
   c->twin->batch_group = c->batch_group;
-  c->twin->pencil_tc = c->pencil_tc;
   c->twin->block_stage = c->block_stage;
-  c->twin->pdl = c->pdl;
   c->twin->spring_len = c->spring_len;
-  // an FP32 schedule chosen by spm_autotune on an FP32 context of this size wins
-  spm_autotune_lookup(c->device, c->N, SPM_FP32, &c->twin->plane_cps, &c->twin->fuse_planes, &c->twin->plane_xg,
-                      &c->twin->pencil_tc, &c->twin->pdl);
+  spm_ctx *t = c->twin;
+  twin_schedule(c, &t->plane_cps, &t->fuse_planes, &t->plane_xg, &t->pencil_tc, &t->pdl);
   return spm_ensure_xg(c->twin);
 }
 

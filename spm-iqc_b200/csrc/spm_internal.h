@@ -65,6 +65,8 @@ struct spm_ctx {
   double spring_len = 0.0;      // SPM spring rest length (0: the reference's zero-length spring)
   spm_ctx *twin = nullptr;      // FP32 twin of an FP64 context (mixed-precision flows)
   void *twin_buf = nullptr;     // FP32 phi and uhat of the twin
+  bool twin_tuned = false;      // the twin's schedule below was chosen by the autotuner
+  int twin_plane_cps = 2, twin_fuse_planes = 1, twin_plane_xg = 0, twin_pencil_tc = 8, twin_pdl = 0;
   const volatile int *cancel = nullptr;  // host flag polled between chunks of steps (job server)
 };
 

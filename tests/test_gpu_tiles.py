@@ -244,3 +244,56 @@ def test_autotuned_choice_does_not_depend_on_the_first_context(cuda):
     assert d.tuning()["pdl"] == c.tuning()["pdl"]
     c.close()
     d.close()
+
+
+def test_autotuning_a_context_tunes_its_fp32_twin(cuda):
+    """spm_autotune on an FP64 context chooses the schedule of the FP32 twin that its
+    mixed flows run on, as it does for an FP32 context; knobs set afterwards win."""
+    import spmiqc
+    N = 128
+    names = ("plane_cps", "fuse_planes", "plane_xg", "pencil_tc", "pdl")
+    get = spmiqc.lib().spm_tune_get
+    get.argtypes = [spmiqc.ctypes.c_void_p, spmiqc.ctypes.c_char_p]
+
+    def twin(c):
+        return {k: int(get(c.h, ("twin_" + k).encode())) for k in names}
+
+    c = spmiqc.SpmContext(N)
+    c.autotune(20)
+    got = twin(c)
+    assert (got["plane_cps"], got["plane_xg"]) in {(1, 0), (2, 0), (3, 0), (2, 1), (2, 2), (2, 3), (3, 3), (4, 3),
+                                                   (5, 3), (6, 3)}
+    d = spmiqc.SpmContext(N, precision="fp32")
+    d.autotune(20)  # the same search, remembered
+    assert d.tuning() == {k: got[k] for k in d.tuning()}
+    # the mixed flow runs with it: the records of an FP32 context of that schedule
+    phi = npo.uniform_field(N, 8)
+    p = cuda.from_numpy(phi.copy()).cuda()
+    st, n32, n64 = c.get_min_u_F_mixed(p, c.my_fft(p), 30, 1e-14, 1e-13)
+    q = cuda.from_numpy(phi).cuda()
+    u = c.my_fft(q)
+    q32, u32 = q.float(), cuda.view_as_real(u).float() if u.is_complex() else u.float()
+    assert (n32, n64) == (30, 0)
+    assert np.array_equal(st, d.get_min_u_F(q32, u32, 30))
+    e = spmiqc.SpmContext(N)
+    e.autotune(20)
+    assert e.tuning() == c.tuning() and twin(e) == got
+    c.close()
+    d.close()
+    e.close()
+
+
+def test_knobs_set_after_tuning_win_over_the_twins_choice(cuda):
+    import spmiqc
+    N = 96  # (no FP32 context of this size is tuned here: its choice would win)
+    get = spmiqc.lib().spm_tune_get
+    get.argtypes = [spmiqc.ctypes.c_void_p, spmiqc.ctypes.c_char_p]
+    c = spmiqc.SpmContext(N)
+    c.autotune(20)
+    for cps in (1, 3):
+        c.tune("plane_cps", cps)
+        assert get(c.h, b"twin_plane_cps") == cps == c.tuning()["plane_cps"]
+    c.autotune(20)
+    assert get(c.h, b"twin_plane_cps") >= 1 and c.tuning()["plane_cps"] == 3
+    assert get(c.h, b"twin_nothing") == -1
+    c.close()
