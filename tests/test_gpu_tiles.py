@@ -297,3 +297,40 @@ def test_knobs_set_after_tuning_win_over_the_twins_choice(cuda):
     assert get(c.h, b"twin_plane_cps") >= 1 and c.tuning()["plane_cps"] == 3
     assert get(c.h, b"twin_nothing") == -1
     c.close()
+
+
+def test_steps_of_extreme_size(cuda):
+    """The step factor 1 / (1 + dt G) beyond the smallest normal number. Both dt = 1e300
+    and dt = 8e307 (denominators up to 1.6e308, factors down to 6e-309) give the
+    spectrum f / G, on the same G (its least value, 2.8e-7, is known to 1e-10 only, so
+    the oracle's is another): they differ by the rounding of the factors, a subnormal
+    number of at least 49 bits, of products, and of the inverse transform, 2^-49 + 30 * 2^-52 < 1e-13
+    of the largest value. A tiny dt leaves the field as it is."""
+    import spmiqc
+    N = 32
+    phi = npo.uniform_field(N, 9)
+    got = {}
+    for dt in (1e300, 8e307, 1e-300):
+        c = spmiqc.SpmContext(N, dt=dt)
+        p = cuda.from_numpy(phi.copy()).cuda()
+        st = c.get_min_u_F(p, c.my_fft(p), 1)
+        assert len(st) == 1 and np.all(np.isfinite(st))
+        got[dt] = p.cpu().numpy()
+        c.close()
+    assert np.max(np.abs(got[1e300])) > 1
+    assert rel(got[8e307], got[1e300]) < 1e-13
+    assert rel(got[1e-300], phi - phi.mean()) < 1e-13
+
+
+def test_preconditioner_with_an_extreme_tau(cuda):
+    """1 / (G + |Tau| + 0.02) with Tau beyond 2^1022, where it is a subnormal number of 50
+    bits: on a field of 1e300 the result is w / Tau minus its mean, to the 1e-13 of the
+    step above."""
+    import spmiqc
+    N = 32
+    w = npo.uniform_field(N, 12, amp=1e300)
+    c = spmiqc.SpmContext(N, Tau=-1e308)
+    got = c.precond_camnew(cuda.from_numpy(w.copy()).cuda()).cpu().numpy()
+    ref = w / 1e308
+    assert rel(got, ref - ref.mean()) < 1e-13
+    c.close()
