@@ -143,8 +143,9 @@ uint64_t spm_launch_count(const spm_ctx *ctx);
  * device code): launches one CTA whose mbarrier wait cannot complete (an
  * arrival expecting 16 bytes with no copy issued) and gives it a limit of
  * `polls` polls of ~256 ns (1 <= polls <= 2^22, the limit every transform
- * kernel's waits use). The wait gives up, sets the context's error word and
- * the kernel returns; the call synchronises the stream and returns what every
+ * kernel's waits use). The wait gives up, another copy that the CTA has in
+ * flight is awaited (its data checked: SPM_ERR_STATE if it is not there), the
+ * context's error word is set and the kernel returns; the call synchronises the stream and returns what every
  * entry point returns after such a timeout: SPM_ERR_CUDA with the message "a
  * kernel's bounded wait for its asynchronous copies timed out". The error
  * word is cleared by that read and the context stays usable. */

@@ -541,6 +541,14 @@ __device__ __forceinline__ bool mbar_wait_n(uint64_t *bar, unsigned parity, int 
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, int *err) {
   return mbar_wait_n(bar, parity, err, kSpinLimit);
 }
+// At the end of a CTA one of whose waits has given up: waits (bounded) until the
+// last of the `issued` copies counted by a barrier has landed, as a copy in
+// flight must not outlive the shared memory that it writes. Once a wait has given
+// up no further copy is issued, so earlier phases are complete.
+__device__ __forceinline__ void drain_copies(uint64_t *bar, int issued) {
+  for (long k = 0; issued > 0 && k < kSpinLimit && !mbar_try_wait(bar, (unsigned)(issued - 1) & 1u); k++)
+    __nanosleep(256);
+}
 
 // ------------------------------------------------------------------ parameters
 struct ModelC {

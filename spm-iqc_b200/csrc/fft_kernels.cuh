@@ -478,7 +478,9 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_fwd_kernel(const __grid_con
   const int cid = blockIdx.x / P::CL, ncl = gridDim.x / P::CL;
   const T *src = reinterpret_cast<const T *>(p.in[b]);
   T2 *dst = reinterpret_cast<T2 *>(p.out[b]);
+  int issued = 0;
   auto issue = [&](int plane) {  // warp 0: one bulk copy per row of this CTA
+    issued++;
     if (lane == 0) mbar_expect_tx(bar, (unsigned)(RW * N * sizeof(T)));
     __syncwarp();
     bulk_g2s(stage + lane * (N / 2), src + ((size_t)plane * N + rank * RW + lane) * N, N * sizeof(T), bar);
@@ -526,7 +528,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_fwd_kernel(const __grid_con
     }
     if (STAGED) __syncthreads();  // every row of the stage is read
     else __syncwarp();
-    if (STAGED && warp == 0 && next < N) {
+    if (STAGED && warp == 0 && next < N && !s_err) {
       fence_proxy_async();
       issue(next);
     }
@@ -537,6 +539,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_fwd_kernel(const __grid_con
     P::template yf<(XG & kXgFwd) != 0>(buf, tw, tid, rank, cluster, dst, plane, xa.first[it & 1]);
     __syncthreads();
   }
+  if (STAGED && tid == 0 && s_err) drain_copies(bar, issued);
   report_error(p, s_err);
   if constexpr (Pro::NR > 0) {
     double tot[Pro::NR];
@@ -617,7 +620,9 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
       cp_async_wait_all();
   };
   // thread 0: two tensor boxes (TC columns x all x) for rows ky0, ky1 of a tile
+  int issued[2] = {0, 0};
   auto issue = [&](const CUtensorMap *map, T2 *dst, uint64_t *bar, int tile) {
+    issued[bar != bars]++;
     const int t = tile / NCH, c0 = (tile % NCH) * TC;
     const int ky0 = t, ky1 = (t == 0) ? N / 2 : N - t;
     mbar_expect_tx(bar, (unsigned)(2 * N * TC * sizeof(T2)));
@@ -691,7 +696,7 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
       }
       if constexpr (USE_SYM) sym_wait();  // this tile's symbols, seen after the barrier
       __syncthreads();
-      if (tid == 0 && next < PG::PTILES) {
+      if (tid == 0 && next < PG::PTILES && !s_err) {
         fence_proxy_async();
         issue(&p.tmi[b], sA, &bars[0], next);
       }
@@ -768,7 +773,7 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
     }
     __syncthreads();  // sS, stab and ex reads done
     if constexpr (Op::SI) {
-      if (tid == 0 && next < PG::PTILES) {
+      if (tid == 0 && next < PG::PTILES && !s_err) {
         fence_proxy_async();
         issue(&p.tms[b], sS, &bars[1], next);
       }
@@ -798,6 +803,8 @@ __global__ void __launch_bounds__(PencilGeo<N, TC>::TH,
       __syncthreads();
     }
   }
+  if (tid == 0 && s_err)
+    for (int i = 0; i < 2; i++) drain_copies(bars + i, issued[i]);
   report_error(p, s_err);
   if constexpr (Op::NR > 0) {
     double tot[Op::NR];
@@ -841,7 +848,9 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_kernel(const __grid_con
   const XgAreas<N, T, RW> xa(p, rank);
   const uint64_t spol = l2_stream_policy();  // streamed field data
   const int cid = blockIdx.x / P::CL, ncl = gridDim.x / P::CL;
+  int issued = 0;
   auto issue = [&](int plane) {  // thread 0: one tensor box (this CTA's 16 columns x all ky)
+    issued++;
     mbar_expect_tx(bar, (unsigned)(N * 16 * sizeof(T2)));
     tma_load_3d(stage, &p.tmi[b], 2 * rank * P::CW, 0, plane, bar);
   };
@@ -874,7 +883,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_kernel(const __grid_con
                         : ld_stream(gsrc + ((size_t)plane * N + ky) * M + rank * P::CW + c, spol);
         },
         xa.own[it & 1]);  // alternating areas, as in plane_fwd
-    if (STAGED && tid == 0 && next < N) {
+    if (STAGED && tid == 0 && next < N && !s_err) {
       fence_proxy_async();
       issue(next);
     }
@@ -896,6 +905,7 @@ __global__ void __launch_bounds__(8 * RW, CPS) plane_inv_kernel(const __grid_con
     }
     __syncthreads();
   }
+  if (STAGED && tid == 0 && s_err) drain_copies(bar, issued);
   report_error(p, s_err);
   if constexpr (Epi::NR > 0) {
     double tot[Epi::NR];

@@ -234,33 +234,52 @@ int spm_check_device_error(spm_ctx *c) {
 
 // The failure path of the bounded waits, run on purpose: one thread arrives
 // on an mbarrier expecting 16 bytes of transactions and no copy is issued, so
-// the phase cannot complete; the wait gives up after `polls` polls, the CTA
-// reports through the context's error word and returns. Nothing is in flight
-// when it returns (no copy was issued), so the context stays usable.
-static __global__ void bounded_wait_selftest_kernel(int *err, long polls) {
-  __shared__ __align__(8) uint64_t bar;
+// the phase cannot complete; the wait gives up after `polls` polls, the CTA lets
+// the copy that it does have in flight land (drain_copies; the context's twiddles, on a
+// barrier that nothing else waits for), reports through the context's error
+// word, with 2 if that copy's data is not there, and returns.
+static __global__ void bounded_wait_selftest_kernel(const int *src, int n, int *err, long polls) {
+  __shared__ __align__(16) int data[1024];
+  __shared__ __align__(8) uint64_t bar[2];
   __shared__ int s_err;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) data[i] = ~src[i];
   if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
     s_err = 0;
     fence_barrier_init();
   }
+  fence_proxy_async();
   __syncthreads();
-  if (threadIdx.x == 0) mbar_expect_tx(&bar, 16);
+  if (threadIdx.x == 0) {
+    mbar_expect_tx(&bar[0], 4u * n);
+    bulk_g2s(data, src, 4u * n, &bar[0]);
+    mbar_expect_tx(&bar[1], 16);
+  }
   __syncthreads();
-  mbar_wait_n(&bar, 0, &s_err, polls);
+  mbar_wait_n(&bar[1], 0, &s_err, polls);
   __syncthreads();
-  if (threadIdx.x == 0 && s_err) atomicExch(err, 1);
+  if (threadIdx.x == 0 && s_err) {
+    drain_copies(&bar[0], 1);
+    int word = 1;
+    for (int i = 0; i < n; i++)
+      if (data[i] != src[i]) word = 2;
+    atomicExch(err, word);
+  }
 }
 
 extern "C" int spm_selftest_bounded_wait(spm_ctx *c, int polls) {
   if (!c || polls < 1 || polls > (int)kSpinLimit) return spm_fail(SPM_ERR_ARG, "polls must be in [1, 2^22]");
   c->launches++;
-  bounded_wait_selftest_kernel<<<1, 32, 0, c->stream>>>(c->flow + FW_ERR, (long)polls);
+  const int n = std::min(1024, c->N * (c->prec == SPM_FP64 ? 4 : 2));  // 32-bit words of the twiddles
+  bounded_wait_selftest_kernel<<<1, 32, 0, c->stream>>>((const int *)c->tw, n, c->flow + FW_ERR, (long)polls);
   cudaError_t e = cudaGetLastError();
+  int word = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&word, c->flow + FW_ERR, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return spm_fail_cuda(e, "bounded-wait self-test");
-  return spm_check_device_error(c);
+  const int rc = spm_check_device_error(c);
+  return word == 2 ? spm_fail(SPM_ERR_STATE, "a copy was still in flight after a bounded wait had given up") : rc;
 }
 
 int spm_read_scal(spm_ctx *c, int nb) {

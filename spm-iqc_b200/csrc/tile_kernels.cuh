@@ -121,20 +121,24 @@ template <int N, class T> constexpr size_t pencil_smem() {
 // The stage shared by a block's G groups: group g has a "full" barrier
 // (completed by the copy's bytes) and an "empty" one (an arrival per warp of the
 // group that has read its tile). The copy of the block's tile i + 1 is issued
-// by the group of tile i once that group has read its own.
+// by the group of tile i once that group has read its own. Once a wait has given
+// up (*err) no copy is issued any more.
 template <int N, int G> struct Stage {
   uint64_t *full, *empty;  // [G]
   int *err;
-  __device__ void init(uint64_t *bars, int *s_err) {
+  volatile int *issued;  // [G] copies issued into `full`; each count has one writer at a time
+  __device__ void init(uint64_t *bars, int *s_ctl) {
     full = bars;
     empty = bars + G;
-    err = s_err;
+    err = s_ctl;
+    issued = s_ctl + 1;
     if (threadIdx.x == 0) {
       for (int g = 0; g < G; g++) {
         mbar_init(full + g, 1);
         mbar_init(empty + g, N / 32);
+        issued[g] = 0;
       }
-      *s_err = 0;
+      *err = 0;
       fence_barrier_init();
     }
   }
@@ -144,11 +148,14 @@ template <int N, int G> struct Stage {
   template <class F> __device__ void next(int g, int tid, int round, F issue) {
     __syncwarp();
     if ((tid & 31) == 0) mbar_arrive(empty + g);
-    if (tid == 0) {
-      mbar_wait(empty + g, round & 1, err);
+    if (tid == 0 && mbar_wait(empty + g, round & 1, err)) {
       fence_proxy_async();
       issue((g + 1) % G);
     }
+  }
+  // At the end, by one thread, once no group issues any more.
+  __device__ void drain() const {
+    for (int g = 0; g < G; g++) drain_copies(full + g, issued[g]);
   }
 };
 
@@ -377,7 +384,7 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
   double *red;
   int g, tid;
   Stage<N, G> st;
-  __device__ PlaneLoop(unsigned char *raw, int *s_err) {
+  __device__ PlaneLoop(unsigned char *raw, int *s_ctl) {
     stage = reinterpret_cast<T2 *>(G > 1 ? smem_base128(raw) : raw);
     tw = stage + PG::STAGE;
     T2 *work = tw + N;
@@ -386,7 +393,7 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
     tid = G > 1 ? threadIdx.x % N : threadIdx.x;
     buf = work + g * PG::UNITS;
     red = reds + g * 32 * kRedMax;
-    if constexpr (G > 1) st.init(reinterpret_cast<uint64_t *>(reds + G * 32 * kRedMax), s_err);
+    if constexpr (G > 1) st.init(reinterpret_cast<uint64_t *>(reds + G * 32 * kRedMax), s_ctl);
   }
   // barrier of the threads that share a tile
   __device__ void sync() const {
@@ -398,6 +405,7 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
     auto issue = [&](int tile, int gg) {
       if constexpr (G > 1) {
         if (tile >= PG::TILES) return;
+        st.issued[gg] = st.issued[gg] + 1;
         mbar_expect_tx(st.full + gg, (unsigned)(PG::STAGE * sizeof(T2)));
         tma_load_4d(stage, &p.tm[b], 0, (tile % P::YB) * N + tile / P::YB, 0, 0, st.full + gg);
       }
@@ -427,6 +435,7 @@ template <int N, class T, bool INV, int G> struct PlaneLoop {
     }
     if constexpr (G > 1) {  // a wait ran out
       __syncthreads();
+      if (*st.err && threadIdx.x == 0) st.drain();
       report_error(p, *st.err);
     }
   }
@@ -477,8 +486,8 @@ __global__ void __launch_bounds__(N, PlaneGeo<N, T>::CPS)
   using P = Plane<N, T>;
   constexpr int N1 = P::N1, YB = P::YB;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_err, s_last[1];
-  PlaneLoop<N, T, false, 1> loop(smem_raw, &s_err);
+  __shared__ int s_last[1];
+  PlaneLoop<N, T, false, 1> loop(smem_raw, nullptr);
   T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
@@ -537,8 +546,8 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
   constexpr int G = inv_groups<N, T>();
   constexpr int N1 = P::N1, YB = P::YB;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_err, s_last[G];
-  PlaneLoop<N, T, true, G> loop(smem_raw, &s_err);
+  __shared__ int s_ctl[1 + G], s_last[G];  // s_ctl: the stage's error word and counts
+  PlaneLoop<N, T, true, G> loop(smem_raw, s_ctl);
   T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
@@ -590,8 +599,8 @@ __global__ void __launch_bounds__(inv_groups<N, T>() * N, PlaneGeo<N, T, inv_gro
   static_assert(NA <= kRedMax, "reduction count");
   constexpr unsigned MAXM = Epi::MAXM | (Pro::MAXM << NE);
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_err, s_last[G];
-  PlaneLoop<N, T, true, G> loop(smem_raw, &s_err);
+  __shared__ int s_ctl[1 + G], s_last[G];  // s_ctl: the stage's error word and counts
+  PlaneLoop<N, T, true, G> loop(smem_raw, s_ctl);
   T2 *const tw = loop.tw, *const buf = loop.buf;
   load_twiddles<N, T>(p, tw);
   grid_dep_sync();
