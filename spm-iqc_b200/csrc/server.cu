@@ -53,8 +53,8 @@ double secs(Clock::time_point a, Clock::time_point b) { return std::chrono::dura
 size_t npts(int N) { return (size_t)N * N * N; }
 
 // Device bytes a job holds while it runs, in fields of N^3 doubles: the
-// job's own arrays, the solver work arrays and the context scratch (two
-// spectral buffers per batched vector), plus the context's tables.
+// job's own arrays, the solver work arrays and the context scratch (a spectral
+// buffer per batched vector, two at least), plus the context's tables.
 size_t footprint_of(const spm_job_desc &d) {
   const double fb = (double)npts(d.N) * (d.precision == SPM_FP32 ? 4 : 8);
   double fields = 0;
@@ -63,13 +63,13 @@ size_t footprint_of(const spm_job_desc &d) {
     case SPM_JOB_RELAX:  // phi, uhat, gradient; scratch 2; FP32 twin: 2 half fields + scratch
       fields = 3 + 2 + (mixed ? 1 + 1 : 0);
       break;
-    case SPM_JOB_LOBPCG: {  // phi, V (k + guard), work 6 per vector, scratch 2 per batched vector
+    case SPM_JOB_LOBPCG: {  // phi, V (k + guard), work 6 per vector, scratch 1 per batched vector (2 at least)
       const double kb = d.k + d.guard;
-      fields = 1 + kb + 6.0 * kb + 2.0 * kb + 1;
+      fields = 1 + kb + 6.0 * kb + kb + 1;
       break;
     }
-    case SPM_JOB_SPM:  // replicas 2, uhat, v/vhat/Gv, scratch 2 x 2; twin half of that
-      fields = 2 + 1 + 3 + 4 + (mixed ? 1 + 3.5 : 0);
+    case SPM_JOB_SPM:  // replicas 2, uhat, v/vhat/Gv, scratch 2; twin: its pair, and half of v/vhat/Gv and scratch
+      fields = 2 + 1 + 3 + 2 + (mixed ? 1 + 2.5 : 0);
       break;
     default: fields = 4;
   }
@@ -77,7 +77,9 @@ size_t footprint_of(const spm_job_desc &d) {
   // autotune in this process: at most 2 x (N x N/32 CTAs) x 16 N FP32 complex
   // values = one FP64 field
   if (mixed) fields += 1;
-  const double tables = (3.0 * (d.N / 2) * (d.N / 2) + 1) * 32 + d.N * 16.0;
+  // factors per |K| and twiddles; FP32 contexts (the twins too) a table over K^2
+  const double k2 = d.precision == SPM_FP64 ? 0.0 : (3.0 * (d.N / 2) * (d.N / 2) + 1) * 16;
+  const double tables = (d.N / 2 + 1) * 16.0 + d.N * 16.0 + k2;
   return (size_t)(fields * fb + tables) + (8u << 20);
 }
 

@@ -88,3 +88,33 @@ def test_cancel_running_job_on_gpu(cuda):
     assert r.status == spmiqc.SPM_ERR_CANCELLED and f is None
     assert r.t_end - r.t_start < 5.0
     assert r2.status == 0
+
+
+@pytest.mark.parametrize("kind,prec", [("relax", "fp64"), ("relax", "mixed"), ("lobpcg", "fp64"), ("spm", "fp64"),
+                                       ("spm", "mixed")])
+def test_footprint_bounds_what_a_job_holds(cuda, kind, prec):
+    """The device memory a running job takes stays within what the scheduler reserves for
+    it, and reservations without the twin's margin are at most 5 % and 16 MB (the
+    allocator's pages and the fixed slack) above it."""
+    import spmiqc
+    N = 160
+    a, b = npo.uniform_field(N, 5), npo.uniform_field(N, 6)
+    desc = spmiqc.job_desc(kind, N, prec, k=8, max_steps=60 if kind == "lobpcg" else 3000, tol=1e-30)
+
+    def run(srv):
+        return srv.submit(desc, a, a + 0.01 * b if kind == "spm" else None)
+
+    with spmiqc.JobServer(max_slots=1) as srv:
+        srv.wait(run(srv))  # kernels are loaded
+        cuda.cuda.synchronize()
+        free0 = low = cuda.cuda.mem_get_info()[0]
+        j = run(srv)
+        end = time.perf_counter() + 60
+        while srv.stats().completed < 2 and time.perf_counter() < end:
+            low = min(low, cuda.cuda.mem_get_info()[0])
+            time.sleep(0.002)
+        assert srv.wait(j)[0].status == 0
+    used, fp = free0 - low, spmiqc.job_footprint(desc)
+    assert 0 < used <= fp, (used, fp)
+    if prec == "fp64":
+        assert fp <= 1.05 * used + (16 << 20), (used, fp)

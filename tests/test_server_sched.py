@@ -200,3 +200,13 @@ def test_serving_stream_is_seeded_and_mixed():
     assert f.shape == (32, 32, 32) and np.isfinite(f).all()
     p0, p1 = workloads.replicas(s, f)
     assert 0.005 < np.max(np.abs(p1 - p0)) <= 0.01 + 1e-12
+
+
+def test_footprint_counts_one_scratch_field_per_vector():
+    """phi, V, six work fields and one scratch field per vector, one to spare; the saddle
+    search's replicas, spectrum, tangent arrays and two scratch fields."""
+    fb, slack = 256 ** 3 * 8, 9 << 20  # slack: tables and small buffers
+    for k in (1, 4, 8):
+        got = job_footprint(job_desc("lobpcg", 256, k=k))
+        assert (1 + 8 * k) * fb <= got <= (2 + 8 * k) * fb + slack
+    assert 8 * fb <= job_footprint(job_desc("spm", 256)) <= 8 * fb + slack
