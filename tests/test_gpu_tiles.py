@@ -334,3 +334,53 @@ def test_preconditioner_with_an_extreme_tau(cuda):
     ref = w / 1e308
     assert rel(got, ref - ref.mean()) < 1e-13
     c.close()
+
+
+def test_block_of_two_at_the_largest_grid(cuda):
+    """256^3 FP64 is where the plane passes copy their tiles through a stage, with a
+    tensor map per field: two different vectors against the oracle, and each alone."""
+    import spmiqc
+    N = 256
+    m = npo.Model(N, L=21.3, Tau=-0.013)
+    c = spmiqc.SpmContext(N, L=21.3, Tau=-0.013)
+    rng = np.random.default_rng(11)
+    phi = 0.1 * rng.standard_normal((N, N, N))
+    v = rng.standard_normal((2, N, N, N))
+    v[1] += 0.25
+    pd, vd = cuda.from_numpy(phi).cuda(), cuda.from_numpy(v).cuda()
+    h = c.hv_cam(pd, vd)
+    for b in range(2):
+        assert cuda.equal(c.hv_cam(pd, vd[b]), h[b])
+        assert rel(h[b].cpu().numpy(), m.hv(phi, v[b])) < 1e-11
+    w = c.precond_camnew(vd).cpu().numpy()
+    for b in range(2):
+        assert rel(w[b], m.precond(v[b])) < 1e-11
+    c.close()
+
+
+@pytest.mark.parametrize("pdl", [0, 1])
+@pytest.mark.parametrize("N", [32, 96, 160, 192])
+def test_fields_alone_and_in_a_block_fused_and_not(cuda, N, pdl):
+    """What acts on the FP64 passes: the number of fields in a launch (single-wave grids
+    let the next launch in, several fields may not), dependent launches, and the joint
+    plane pass. The same bits."""
+    import spmiqc
+    phi = npo.uniform_field(N, 21)
+    V = cuda.from_numpy(np.stack([npo.uniform_field(N, 70 + i, amp=1.0) for i in range(3)])).cuda()
+    out = []
+    for fuse in (0, 1):
+        c = spmiqc.SpmContext(N, Tau=-0.02)
+        c.tune("pdl", pdl)
+        c.tune("fuse_planes", fuse)
+        p = cuda.from_numpy(phi.copy()).cuda()
+        u = c.my_fft(p)
+        st = c.get_min_u_F(p, u, 11)
+        h = c.hv_cam(p, V)
+        w = c.precond_camnew(V.clone())
+        for b in range(3):
+            assert cuda.equal(c.hv_cam(p, V[b]), h[b])
+            assert cuda.equal(c.precond_camnew(V[b].clone()), w[b])
+        out.append((st, p, u, h, w))
+        c.close()
+    (s0, *a), (s1, *b) = out
+    assert np.array_equal(s0, s1) and all(cuda.equal(x, y) for x, y in zip(a, b))
