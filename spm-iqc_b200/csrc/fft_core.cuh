@@ -687,7 +687,7 @@ struct SymFn {
   double g;
   double pre;  // the scalar that an operator with PRE reads (pencil_kernel), else 0
   __device__ double G() const { return g; }
-  // 1/(1 + dt G) and the preconditioner's 1/(G + |Tau| + 0.02) come from an eighth of
+  // 1/(1 + dt G) and the preconditioner's 8/(G + |Tau| + 0.02) come from an eighth of
   // the denominator (exact, folded into its terms), so that no finite dt or Tau is
   // beyond the range in which the approximation is normal; a result below 2^-1022
   // is rounded once, at the end. A zero denominator (dt < 0) gives the
@@ -696,9 +696,9 @@ struct SymFn {
     const double x8 = fma(0.125 * m.dt, g, 0.125), y = rcp_approx(x8), r = 0.125 * rcp_refine(x8, y);
     return (__double2hiint(y) & 0x7fffffff) == 0x7ff00000 ? y : r;
   }
-  __device__ double prec(const ModelC &m) const {
+  __device__ double prec8(const ModelC &m) const {
     const double x8 = fma(0.125, g, 0.125 * fabs(m.Tau)) + 0.125 * 0.02;
-    return 0.125 * rcp_refine(x8, rcp_approx(x8));
+    return rcp_refine(x8, rcp_approx(x8));
   }
   __device__ double force() const { return rcp_refine(1.0 + g, rcp_approx(1.0 + g)); }
   __device__ static double scale(const ModelC &m) { return m.fscale; }

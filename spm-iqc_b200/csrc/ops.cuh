@@ -296,8 +296,8 @@ template <class T> struct OpPrecond {
   template <class S>
   __device__ static void point(const KParams &p, int, int Kx, int Ky, int Kz, S sy, c2<T> f, c2<T>, c2<T> &,
                                c2<T> &inv, double (&)[1], double) {
-    const T ik = (T)sy.prec(p.m);  // 1 / (G + |Tau| + 0.02)
-    inv = cscale(cscale(f, (T)S::scale(p.m)), ik);
+    const T ik8 = (T)sy.prec8(p.m);  // 8 / (G + |Tau| + 0.02); the eighth is in the scale
+    inv = cscale(cscale(f, (T)(0.125 * S::scale(p.m))), ik8);
   }
   __device__ static void fin(const KParams &, int, const double (&)[1]) {}
 };
