@@ -116,8 +116,8 @@ const char *spm_status_str(int status);
  * programmatic dependents (in a stream capture, programmatic edges of the
  * graph): a launch may be set up while the previous kernel of the stream
  * completes, and its kernel waits on the device for that kernel before its
- * first memory access; 0 (default) = plain stream order. The same bits
- * either way; spm_autotune turns it on where it is at least 1 % faster.
+ * first memory access; 0 (default) = plain stream order, except that grids
+ * of one wave are launched that way in any case. The same bits either way; spm_autotune turns it on where it is at least 1 % faster.
  * spm_tune_get returns the current value or -1 for an unknown knob; on FP64
  * contexts "twin_" before a name (twin_plane_cps, twin_fuse_planes, twin_plane_xg,
  * twin_pencil_tc, twin_pdl) gives what the FP32 twin of mixed runs takes: the

@@ -2,10 +2,10 @@
 // sizes and parameters), advanced by rounds of `steps_per_launch` gated steps of
 // every instance. Instances of the
 // same grid size and precision form groups of up to 16 that share every
-// launch (one launch per pass for the whole group, blockIdx.y = instance,
+// launch (one launch per pass for the whole group,
 // each instance with its own model, symbols and flow words); each group runs
 // on its own stream, so groups of different sizes overlap on the
-// device. (With the context knob "batch_group" = 0 on the first instance,
+// device; long runs of several groups go through a captured graph. (With the context knob "batch_group" = 0 on the first instance,
 // every instance gets its own stream and launches instead.) Instances stop
 // on the device (convergence or their step cap); rounds are launched until
 // every instance has stopped. With switch_tol > 0 the instances first run on
@@ -95,7 +95,7 @@ int group_steps(spm_ctx *const *ctx, void *const *phi, void *const *uh, const st
 }
 
 // Runs the flows of n contexts to tol (or max_steps each); steps[i] += done.
-// With stall > 0 an instance is also stopped (between graph launches) once
+// With stall > 0 an instance is also stopped (between rounds) once
 // FloorWatch (windows of `stall` steps, switch point tol) sees its FP32
 // rounding floor.
 // caps (may be null) gives each instance its own step budget (<= max_steps).

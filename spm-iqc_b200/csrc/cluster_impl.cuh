@@ -1,11 +1,12 @@
 // Kernel chains over the cluster passes (fft_kernels.cuh): the FP32 gradient
 // chains, transforms, energy and gradient. They stay beside the tile passes
-// (ops_impl.cuh) because an FP32 flow's FP64 step records (energy, residual,
-// gradient norm), which callers compare to 1e-9, follow the FP32 rounding of
-// every transform value: the tile passes factor the transforms differently,
-// which moves those records by about 3e-7 relative (the fields by as much as
-// any two FP32 transforms differ). At 256^3 an FP32 step takes 186 us here; the
-// tile passes took 214 us with four-column runs and the spectrum in the caller's order.
+// (ops_impl.cuh) so that FP32 flows keep giving the step records that they gave
+// before: the records (energy, residual, gradient norm) are FP64 numbers that follow
+// the FP32 rounding of every transform value, and the tile passes factor the
+// transforms differently, which moves them by about 3e-7 relative. (An FP32 flow
+// is about 1e-6 from its 64-bit values either way.) At 256^3 an FP32 step takes
+// 184-194 us here; the tile passes took 214 us with the spectrum in the caller's order, and
+// have not been timed for FP32 chains with it in tile order.
 #pragma once
 
 #include "blas1.cuh"
@@ -87,7 +88,7 @@ static inline int eff_cps(const spm_ctx *c) { return cps_rw16(c) ? 2 : c->plane_
 static inline int xg_bits(const spm_ctx *c, int nb) { return (c->xg && nb == 1 && eff_cps(c) >= 2) ? c->plane_xg : 0; }
 static inline bool rw16(const spm_ctx *c, int nb) { return cps_rw16(c) && xg_bits(c, nb) == (kXgFwd | kXgInv); }
 // Four CTAs per SM (64 registers per thread): FP32 gradient chains only.
-template <class T> static inline bool cps4(const spm_ctx *c) { return sizeof(T) == 4 && eff_cps(c) == 4; }
+static inline bool cps4(const spm_ctx *c) { return eff_cps(c) == 4; }
 
 // The plane kernels come in four variants (c->plane_cps): 1 = staged, one CTA
 // per SM; 2 = direct loads, two CTAs per SM; 3 = direct, three CTAs per SM;
@@ -100,12 +101,10 @@ template <int N, class T, class Pro> static int plane_fwd(spm_ctx *c, KParamsC &
         return launch_cluster<Tag16, N, decltype(&plane_fwd_kernel<N, T, Pro, 4, kXgFwd, 16>), 16>(
             c, plane_fwd_kernel<N, T, Pro, 4, kXgFwd, 16>, plane_smem<N, T, 4, 16>(), p, nb, "plane_fwd", true);
       }
-      if constexpr (sizeof(T) == 4) {
-        if (cps4<T>(c)) {
-          struct Tag4x {};
-          return launch_cluster<Tag4x, N>(c, plane_fwd_kernel<N, T, Pro, 4, kXgFwd>, plane_smem<N, T, 4>(), p, nb,
-                                          "plane_fwd", true);
-        }
+      if (cps4(c)) {
+        struct Tag4x {};
+        return launch_cluster<Tag4x, N>(c, plane_fwd_kernel<N, T, Pro, 4, kXgFwd>, plane_smem<N, T, 4>(), p, nb,
+                                        "plane_fwd", true);
       }
       if (eff_cps(c) >= 3) {
         struct Tag3x {};
@@ -136,12 +135,10 @@ template <int N, class T, class Epi> static int plane_inv(spm_ctx *c, KParamsC &
         return launch_cluster<Tag16, N, decltype(&plane_inv_kernel<N, T, Epi, 4, kXgInv, 16>), 16>(
             c, plane_inv_kernel<N, T, Epi, 4, kXgInv, 16>, plane_smem<N, T, 4, 16>(), p0, nb, "plane_inv", true);
       }
-      if constexpr (sizeof(T) == 4) {
-        if (cps4<T>(c)) {
-          struct Tag4x {};
-          return launch_cluster<Tag4x, N>(c, plane_inv_kernel<N, T, Epi, 4, kXgInv>, plane_smem<N, T, 4>(), p0, nb,
-                                          "plane_inv", true);
-        }
+      if (cps4(c)) {
+        struct Tag4x {};
+        return launch_cluster<Tag4x, N>(c, plane_inv_kernel<N, T, Epi, 4, kXgInv>, plane_smem<N, T, 4>(), p0, nb,
+                                        "plane_inv", true);
       }
       if (eff_cps(c) >= 3) {
         struct Tag3x {};
@@ -170,8 +167,8 @@ template <int N, class T, class Epi> static int plane_inv(spm_ctx *c, KParamsC &
 // three with plane_cps = 3), with the exchange routes XG.
 template <int N, class T, class Epi, class Pro, int XG>
 static int plane_inv_fwd_xg(spm_ctx *c, KParamsC &p, int nb) {
-  if constexpr (sizeof(T) == 4 && XG != 0) {
-    if (cps4<T>(c)) {
+  if constexpr (XG != 0) {
+    if (cps4(c)) {
       struct Tag4 {};
       return launch_cluster<Tag4, N>(c, plane_inv_fwd_kernel<N, T, Epi, Pro, 4, XG>, plane_smem<N, T, 4>(), p, nb,
                                      "plane_inv_fwd", true);
@@ -257,6 +254,7 @@ template <int N, class T, class Op> static int pencil(spm_ctx *c, KParamsC &p, i
   return pencil_tc<N, T, Op, 8>(c, p, nb);
 }
 template <int N, class T> struct Chains {
+  static_assert(sizeof(T) == 4, "the cluster passes serve FP32 contexts");
   static int fft(spm_ctx *c, const void *x, void *xhat) {
     SPM_NEED_SCRATCH(c, 2);
     KParamsC p = spm_params_c(c);

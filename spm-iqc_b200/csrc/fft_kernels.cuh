@@ -90,7 +90,7 @@ template <int N, class T, int TC = 8> constexpr int pencil_min_ctas(int stages, 
     const int k = smem_ctas_per_sm(pencil_smem_n<N, T, TC>(stages, pencil_sym_bufs<N, T, TC>(stages, sym)));
     return k < 1 ? 1 : (k > 4 ? 4 : k);
   } else {
-    return sizeof(T) == 4 && smem_ctas_per_sm(pencil_smem_n<N, T>(stages, sym ? 1 : 0)) >= 2 ? 2 : 1;
+    return smem_ctas_per_sm(pencil_smem_n<N, T>(stages, sym ? 1 : 0)) >= 2 ? 2 : 1;
   }
 }
 template <int N, class T, int TC = 8> constexpr size_t pencil_smem(int stages, bool sym) {

@@ -119,6 +119,8 @@ template <int N, class T> struct Impl {
     p.in[0] = phi;
     p.st[0] = uhat;
     c->launches++;
+    // blocks: eight per SM, or two, get_Ene with its read-back: 32^3 42.3 / 41.7, 64^3 and
+    // 96^3 equal, 128^3 42.0 / 43.5, 192^3 65 / 91, 256^3 111 / 172 us
     energy_kernel<T><<<N >= 128 ? kReduceBlocks : kReduceBlocks / 4, kThreads, 0, c->stream>>>(p, N);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : spm_fail_cuda(e, "energy");
@@ -145,7 +147,7 @@ template <int N, class T> struct Impl {
 
   // The passes of a gradient chain over n instances of this grid size and
   // precision (ctx, phi, uhat: arrays of n), one launch per pass for all of
-  // them (blockIdx.y = instance). Each instance keeps its own fields, scratch,
+  // them (field_id() = instance). Each instance keeps its own fields, scratch,
   // model, symbol factors, flow words and step records; the partial sums,
   // tickets and scalars use one slot per instance in ctx[0]'s buffers, and
   // ctx[0]'s stream and tuning serve the launches. A stopped instance's blocks

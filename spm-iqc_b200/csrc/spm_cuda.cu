@@ -167,7 +167,7 @@ int spm_tensor_map(spm_ctx *c, const void *ptr, int kind, CUtensorMap *out) {
   auto fn = encode_fn();
   if (!fn) return spm_fail(SPM_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
   const int N = c->N;
-  const size_t es = c->prec == SPM_FP64 ? 8 : 4;
+  constexpr size_t es = 4;  // FP32 contexts only (cluster passes)
   const cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)N, (cuuint64_t)N};  // N reals = N/2 complex per row
   const cuuint64_t strides[2] = {(cuuint64_t)N * es, (cuuint64_t)N * N * es};
   cuuint32_t box[3];
@@ -184,7 +184,7 @@ int spm_tensor_map(spm_ctx *c, const void *ptr, int kind, CUtensorMap *out) {
   TmEntry e;
   e.ptr = ptr;
   e.kind = kind;
-  CUresult r = fn(&e.map, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+  CUresult r = fn(&e.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                   const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return spm_fail(SPM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
